@@ -230,16 +230,19 @@ __global__ void k_dist2d_query(DevEnv E, int cdf_mode, const float* __restrict__
 // reads a hit's normals with three loads from one 48-B record that does not
 // wait for the instance, instead of a vertex-id record and nine loads that
 // wait on it (shade 43.5 against 44.7 ms on the 1080p studio frame).
-__global__ void k_slot_normals(const float4* __restrict__ tris, const uint32_t* __restrict__ index,
+// The same pass writes into the triangle record the slot of the one static
+// instance that uses its mesh (-1: none, or several).
+__global__ void k_slot_normals(float4* __restrict__ tris, const uint32_t* __restrict__ index,
                                const float* __restrict__ normal, const uint32_t* __restrict__ slot_start,
                                const uint32_t* __restrict__ index_base, const uint8_t* __restrict__ has_normals,
-                               uint32_t n_mesh, uint32_t n_slots, float4* __restrict__ out) {
+                               const int32_t* __restrict__ inst_of, uint32_t n_mesh, uint32_t n_slots, float4* __restrict__ out) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n_slots; t += gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = n_mesh - 1;  // last mesh with slot_start <= t
         while (lo < hi) {
             const uint32_t mid = (lo + hi + 1) / 2;
             if (slot_start[mid] <= t) lo = mid; else hi = mid - 1;
         }
+        tris[3 * (size_t)t + 1].w = __int_as_float(inst_of[lo]);
         const size_t row = index_base[lo] + 3 * (size_t)__float_as_uint(tris[3 * (size_t)t].w);
         for (int k = 0; k < 3; ++k) {
             float4 n = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -250,6 +253,77 @@ __global__ void k_slot_normals(const float4* __restrict__ tris, const uint32_t* 
             out[3 * (size_t)t + k] = n;
         }
     }
+}
+
+// GpuNodes to trace nodes, in place (layout and visiting order:
+// device_scene.cuh, "binary traversal"). Nodes below top_base belong to
+// instance BVHs, the others to the top level. The last triangle of each leaf
+// gets its mark. An empty child (the second of a one-leaf BVH) becomes a LEAVE
+// entry, which does nothing there, behind a box that no ray meets unless its
+// direction is exactly along (1, 2, 4).
+__global__ void k_pack_nodes(GpuNode* __restrict__ nodes, uint32_t n_nodes, uint32_t top_base,
+                             const DevInstance* __restrict__ inst, float4* __restrict__ tris) {
+    enum { INTERIOR, LEAF, ENTRY, EMPTY };
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x) {
+        const GpuNode g = nodes[i];
+        float4 out[4];
+        float* f = reinterpret_cast<float*>(out);
+        int ref[2], kind[2];
+        uint32_t counts = 0;
+        for (int s = 0; s < 2; ++s) {
+            const float* xy = s == 0 ? g.a : g.b;  // lo.x, hi.x, lo.y, hi.y
+            const int32_t child = g.d[s], count = g.d[2 + s];
+            float lo[3] = {xy[0], xy[2], g.c[2 * s]}, hi[3] = {xy[1], xy[3], g.c[2 * s + 1]};
+            if (child < 0) {
+                kind[s] = EMPTY;
+                ref[s] = PYRE_REF_LEAVE;
+                for (int c = 0; c < 3; ++c) lo[c] = hi[c] = 1e30f * (float)(1 << c);
+            } else if (count == 0) {
+                kind[s] = INTERIOR;
+                ref[s] = child;
+            } else if (i < top_base) {
+                kind[s] = LEAF;
+                ref[s] = PYRE_REF_LEAF | child;
+                counts |= (uint32_t)count << (16 * s);
+                tris[3 * (size_t)(child + count - 1) + 2].w = __uint_as_float(1u);
+            } else {
+                const int32_t k = count > 0 ? child : child & ~(PYRE_TAG_INST | PYRE_TAG_TOP);
+                const bool direct = count < 0 && inst[k].direct;
+                kind[s] = direct ? INTERIOR : ENTRY;
+                ref[s] = direct ? inst[k].blas_root : PYRE_REF_INST | k;
+            }
+            f[4 * s] = lo[0]; f[4 * s + 1] = lo[1]; f[4 * s + 2] = hi[0]; f[4 * s + 3] = hi[1];
+            f[8 + 2 * s] = lo[2]; f[9 + 2 * s] = hi[2];
+        }
+        float bias = 0.0f;
+        if (kind[0] != INTERIOR || kind[1] != INTERIOR) {
+            const bool second = kind[0] != LEAF && (kind[1] == LEAF || (kind[0] == ENTRY && kind[1] == INTERIOR));
+            bias = second ? INFINITY : -INFINITY;
+        }
+        f[12] = __int_as_float(ref[0]); f[13] = __int_as_float(ref[1]);
+        f[14] = bias; f[15] = __uint_as_float(counts);
+        float4* w = reinterpret_cast<float4*>(nodes + i);
+        for (int q = 0; q < 4; ++q) w[q] = out[q];
+    }
+}
+
+// A trace node of an instance BVH back as the GpuNode it was packed from.
+GpuNode unpack_node(const GpuNode& packed) {
+    float f[16];
+    std::memcpy(f, &packed, sizeof f);
+    GpuNode g;
+    uint32_t counts;
+    std::memcpy(&counts, &packed.d[3], 4);
+    for (int s = 0; s < 2; ++s) {
+        const int32_t ref = packed.d[s];
+        Aabb b;
+        b.lo = mk3(f[4 * s], f[4 * s + 1], f[8 + 2 * s]);
+        b.hi = mk3(f[4 * s + 2], f[4 * s + 3], f[9 + 2 * s]);
+        if (ref >= 0) set_gpu_child(g, s, b, ref, 0);
+        else if (ref == PYRE_REF_LEAVE) set_gpu_child(g, s, b, -1, 0);
+        else set_gpu_child(g, s, b, ref & PYRE_REF_SLOT, (int32_t)((counts >> (16 * s)) & 0xffffu));
+    }
+    return g;
 }
 
 // BsdfSample / eval / pdf (material.rs:42-226) per (wo, u): out gets
@@ -490,6 +564,12 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
 
     // ---- instances and one top-level BVH per part over their swept bounds
     std::vector<DevInstance> inst;
+    std::vector<uint32_t> mesh_users(n_meshes, 0);    // instances per mesh
+    std::vector<int32_t> mesh_inst(n_meshes, -1);     // slot of the one static instance of a mesh
+    std::vector<int32_t> more;                        // slots followed by another of their top-level leaf
+    for (uint32_t i = 0; i < desc->n_instances; ++i) mesh_users[desc->instances[i].mesh] += 1;
+    sc->top_base = node_off + (int32_t)nodes.size();
+    const size_t first_top_node = nodes.size();
     std::vector<int32_t> part_tlas(n_parts, -1);
     sc->slot_of_instance.assign(desc->n_instances, -1);
     for (uint32_t part = 0; part < n_parts; ++part) {
@@ -525,7 +605,7 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
         if (live.empty()) continue;
         std::vector<pyre_bvh2_node> tn;
         std::vector<uint32_t> tp;
-        build_bvh2(ibox, icent, tn, tp, PYRE_TLAS_ENTER ? 1u : 8u);
+        build_bvh2(ibox, icent, tn, tp, 1u);
         const int32_t slot_base = (int32_t)inst.size();
         part_tlas[part] = node_off + (int32_t)nodes.size();
         const size_t first_top = nodes.size();
@@ -534,8 +614,9 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
         // box, unpadded, and the child entry INST|TOP|slot with count -1: the
         // top-level step's test of the box is the reference's root test
         // (bvh.rs:103-110) and the lane then enters the instance without a
-        // node step of its own.
-        for (size_t g = first_top; PYRE_TLAS_ENTER && g < nodes.size(); ++g)
+        // node step of its own. Where no other instance uses the mesh, the
+        // binary traversal has no entry at all (k_pack_nodes).
+        for (size_t g = first_top; g < nodes.size(); ++g)
             for (int c = 0; c < 2; ++c) {
                 if (nodes[g].d[2 + c] != 1) continue;
                 const int32_t slot = nodes[g].d[c];
@@ -544,6 +625,8 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
                 set_gpu_child(nodes[g], c, mesh_box[id.mesh], slot | PYRE_TAG_INST | PYRE_TAG_TOP, -1);
             }
         inst.resize(inst.size() + tp.size());
+        for (const pyre_bvh2_node& nd : tn)  // leaves of several instances (coincident centroids)
+            for (uint32_t k = 1; k < nd.n_primitives; ++k) more.push_back(slot_base + (int32_t)(nd.offset + k - 1));
         for (size_t k = 0; k < tp.size(); ++k) {
             uint32_t i = live[tp[k]];
             const pyre_instance_desc& id = desc->instances[i];
@@ -556,14 +639,20 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
             I.has_motion = id.has_motion ? 1 : 0;
             for (int c = 0; c < 3; ++c) { I.off0[c] = id.offset_t0[c]; I.off1[c] = id.offset_t1[c]; }
             I.orig_id = (int32_t)i;
-            I.mesh = (int32_t)id.mesh;
+            I.direct = !id.has_motion && mesh_users[id.mesh] == 1 ? 1u : 0u;
+            if (I.direct) mesh_inst[id.mesh] = slot_base + (int32_t)k;
             I.material = id.material;
             I.index_base = (uint32_t)mesh_index_base[id.mesh];
             I.normal_base = mesh_normal_base[id.mesh];
-            I.tri_count = desc->meshes[id.mesh].n_triangles;
             sc->slot_of_instance[i] = slot_base + (int32_t)k;
         }
     }
+    for (int32_t k : more) inst[(size_t)k].more = 1;
+    // the top level as it is, for the wide traversals (node indices from 0)
+    sc->top.assign(nodes.begin() + (std::ptrdiff_t)first_top_node, nodes.end());
+    for (GpuNode& g : sc->top)
+        for (int c = 0; c < 2; ++c)
+            if (g.d[2 + c] == 0 && g.d[c] >= 0) g.d[c] -= sc->top_base;
     const int32_t tlas_root = part_tlas[0];
     // per-part light ranges (first, count)
     std::vector<uint32_t> part_light(2 * n_parts, 0);
@@ -645,6 +734,7 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
     D.slot_normals = nullptr;
     if (total_tris) {
         std::vector<uint32_t> slot_start, index_base;
+        std::vector<int32_t> inst_of;
         std::vector<uint8_t> has_normals;
         uint32_t acc = 0;
         for (uint32_t m = 0; m < n_meshes; ++m) {
@@ -652,13 +742,16 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
             slot_start.push_back(acc);
             index_base.push_back((uint32_t)mesh_index_base[m]);
             has_normals.push_back(mesh_normal_base[m] >= 0 ? 1 : 0);
+            inst_of.push_back(mesh_inst[m]);
             acc += desc->meshes[m].n_triangles;
         }
         uint32_t *d_start = nullptr, *d_base = nullptr;
+        int32_t* d_inst_of = nullptr;
         uint8_t* d_has = nullptr;
         if ((rc = upload(ctx, sc, slot_start, &d_start)) != PYRE_OK) return fail(rc);
         if ((rc = upload(ctx, sc, index_base, &d_base)) != PYRE_OK) return fail(rc);
         if ((rc = upload(ctx, sc, has_normals, &d_has)) != PYRE_OK) return fail(rc);
+        if ((rc = upload(ctx, sc, inst_of, &d_inst_of)) != PYRE_OK) return fail(rc);
         void* p = nullptr;
         if (injected_alloc_failure(ctx))
             return fail(set_error(ctx, PYRE_ERR_OOM, "cudaMalloc(scene): injected allocation failure"));
@@ -667,8 +760,11 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
         sc->allocations.push_back(p);
         sc->device_bytes += (size_t)total_tris * 3 * sizeof(float4);
         const uint32_t grid = (uint32_t)std::min<uint64_t>((total_tris + 255) / 256, 65535);
-        k_slot_normals<<<grid, 256>>>(d_tris, d_index, d_normal, d_start, d_base, d_has, (uint32_t)slot_start.size(),
-                                      (uint32_t)total_tris, (float4*)p);
+        k_slot_normals<<<grid, 256>>>(d_tris, d_index, d_normal, d_start, d_base, d_has, d_inst_of,
+                                      (uint32_t)slot_start.size(), (uint32_t)total_tris, (float4*)p);
+        const uint64_t n_nodes = (uint64_t)node_off + nodes.size();
+        k_pack_nodes<<<(uint32_t)std::min<uint64_t>((n_nodes + 255) / 256, 65535), 256>>>(
+            d_nodes, (uint32_t)n_nodes, (uint32_t)sc->top_base, d_inst, d_tris);
         e = cudaDeviceSynchronize();
         if (e == cudaSuccess) e = cudaGetLastError();
         if (e != cudaSuccess) return fail(cuda_check(ctx, e, "slot normals"));
@@ -729,13 +825,14 @@ int select_bvh(pyre_ctx* ctx, pyre_scene* scene, uint32_t requested, DevScene* d
             return set_error(ctx, PYRE_ERR_INVALID, "the scene has no width-" + std::to_string(w) +
                                                         " BVH yet (pyre_scene_set_bvh_width builds it)");
         // collapse from the binary device BVH: one wide BVH per distinct instance BVH
-        std::vector<GpuNode> bin(scene->n_nodes);
+        std::vector<GpuNode> bin((size_t)scene->top_base);
         std::vector<DevInstance> inst(scene->dev.n_inst);
         PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
         PYRE_CUDA_TRY(ctx, cudaMemcpy(bin.data(), scene->dev.nodes, bin.size() * sizeof(GpuNode),
                                       cudaMemcpyDeviceToHost));
         PYRE_CUDA_TRY(ctx, cudaMemcpy(inst.data(), scene->dev.inst, inst.size() * sizeof(DevInstance),
                                       cudaMemcpyDeviceToHost));
+        for (GpuNode& g : bin) g = unpack_node(g);
         std::vector<float> flat;
         std::map<int32_t, int32_t> wide_of;
         std::vector<int32_t> roots(inst.size(), -1);
@@ -753,11 +850,14 @@ int select_bvh(pyre_ctx* ctx, pyre_scene* scene, uint32_t requested, DevScene* d
         std::memcpy(nodes4.data(), flat.data(), flat.size() * sizeof(float));
         int rc = upload(ctx, scene, nodes4, &wd.nodes);
         if (!rc) rc = upload(ctx, scene, roots, &wd.root);
+        if (!rc && !scene->d_top) rc = upload(ctx, scene, scene->top, &scene->d_top);
         if (rc) { wd.nodes = nullptr; wd.root = nullptr; return rc; }
         wd.n_nodes = n_wide;
     }
     dev->wnodes = wd.nodes;
     dev->wroot = wd.root;
+    dev->nodes = reinterpret_cast<const float4*>(scene->d_top);
+    dev->tlas_root = scene->top_root(0);
     return PYRE_OK;
 }
 

@@ -1,10 +1,13 @@
 // device_scene.cuh — scene layout in HBM and ray traversal (closest / any hit).
 //
 // Layout (all arrays device-resident, built once by pyre_scene_upload):
-//   nodes  GpuNode[]    64-B binary nodes: every mesh BVH (collapsed from the
-//                       reference BVH2), then the top-level BVH over instances
+//   nodes               64-B trace nodes (see "binary traversal" below): every
+//                       mesh BVH (collapsed from the reference BVH2), then the
+//                       top-level BVH over instances
 //   tris   float4[3*T]  per triangle slot, in BVH leaf order:
-//                       (v0.xyz, original triangle id as bits), (e1.xyz, 0), (e2.xyz, 0)
+//                       (v0.xyz, original triangle id as bits),
+//                       (e1.xyz, instance slot as bits, -1 where several instances use the mesh),
+//                       (e2.xyz, 1 as bits in the last triangle of a leaf)
 //                       with e1 = v1 - v0, e2 = v2 - v0 rounded exactly as
 //                       moller_trumbore computes them (mesh.rs:153-157)
 //   inst   DevInstance[] instances in top-level-leaf order
@@ -29,11 +32,11 @@ struct alignas(16) DevInstance {
     float off0[3];
     int32_t orig_id;    // index in Scene::primitives
     float off1[3];
-    int32_t mesh;
+    int32_t more;       // the top-level leaf holds the next slot too
     uint32_t material;
     uint32_t index_base;   // first index (3 per triangle) of the mesh in `index`
     int32_t normal_base;   // first vertex of the mesh's normals, -1 if none
-    uint32_t tri_count;
+    uint32_t direct;       // static, and no other instance uses its mesh: its root hangs below the top level
 };
 
 struct alignas(16) DevMaterial {
@@ -79,9 +82,10 @@ struct DevScene {
     const int32_t* part_tlas;    // top-level root per part
     const uint32_t* part_light;  // (first light, light count) per part
     uint32_t n_parts;
-    // wide BVH of the instances (traversals with WIDTH 4 or 8; the top level
-    // stays binary): wide nodes (8 fields x WIDTH floats each) and the wide
-    // root of each instance slot
+    // wide BVH of the instances (traversals with WIDTH 4 or 8): wide nodes (8
+    // fields x WIDTH floats each) and the wide root of each instance slot. The
+    // top level stays binary; for these traversals `nodes` holds it alone, as
+    // GpuNodes with instance entries
     const float4* wnodes;
     const int32_t* wroot;
 };
@@ -101,38 +105,27 @@ struct TraceHit {
 
 #define PYRE_STACK 64
 // lanes of a warp that may still be looking for a leaf when the leaf phase
-// starts, for closest-hit and any-hit traversal
-// (with two node steps per vote: 12 and 16 against 8 and 12 gave 702.0 and
-// 702.7 against 701.0 Msamples/s one at a time; 6 and 8 gave 696.5 and 696.8.
-// With instances entered from the top-level step and 9 closest-hit blocks,
-// 10 closest-hit lanes measured 748.3 against 746.2 for 12, and 8 748.1.
-// Once closest-hit lanes stopped at their first leaf, 16 lanes measured
-// 758.8 against 755.6 for 10, 750.7 for 20 and 741.1 for 24)
+// starts, for closest-hit and any-hit traversal: 12 / 16 / 20 gave 127.1 /
+// 126.9 / 128.0 ms per 1080p studio frame and 2.88 / 2.90 / 3.00 ms on the
+// closest-hit microbenchmark
 #ifndef PYRE_LEAF_WAIT_CLOSEST
 #define PYRE_LEAF_WAIT_CLOSEST 16
 #endif
 #ifndef PYRE_LEAF_WAIT_ANY
 #define PYRE_LEAF_WAIT_ANY 16
 #endif
-// Node steps a lane takes between two warp votes of the inner phase. Each
-// vote (a ballot, a population count and an any) costs issue slots; taking
-// two steps per vote measured 701.8 against 681.0 Msamples/s on the 1080p
-// studio frame (extend 104.0 against 109.4 ms), three 700.6. With instances
-// entered from the top-level step, three measured 751.3 against 746.4 for
-// two (extend 93.9 against 94.9 ms); with 256-bit node loads, four measured
-// 768.5 against 763.4 for three. Films are bit-identical for every setting.
+// Node steps a lane takes between two warp votes of the inner phase (a vote, a
+// ballot, a population count and an any, costs issue slots): 3 / 4 / 6 gave
+// 127.5 / 126.9 / 126.6 ms per 1080p studio frame and 2.93 / 2.90 / 2.87 ms on
+// the closest-hit microbenchmark. Films are bit-identical for every setting.
 #ifndef PYRE_STEPS_PER_VOTE
-#define PYRE_STEPS_PER_VOTE 4
+#define PYRE_STEPS_PER_VOTE 6
 #endif
 
-// Binary node fetch: one 64-B node as two 256-bit loads (sm_100+ `ld.v8`;
-// nodes are 64-B aligned) instead of four 128-bit ones, so a node step issues
-// two load instructions. The traversal is issue-bound: 763.4 against 749.8
-// Msamples/s on the 1080p studio frame (extend 92.1 against 94.0 ms, shadow
-// 33.2 against 34.5 ms), films bit-identical.
-#ifndef PYRE_LD256
-#define PYRE_LD256 1
-#endif
+// 32 B with one load (sm_100+; p is 32-B aligned). A traversal step fetches
+// its 64-B node with two of these instead of four 128-bit loads: 763.4 against
+// 749.8 Msamples/s on the 1080p studio frame, the traversal being bound by
+// instruction issue.
 __device__ __forceinline__ void ldg_256(const float4* p, float4& a, float4& b) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -192,55 +185,336 @@ __device__ __forceinline__ f3 motion_offset(const DevInstance& I, float time) {
                  clampf_(time, 0.0f, 1.0f));
 }
 
-// Warp-synchronous two-level traversal (top-level BVH over instances, then
-// each reached instance's BVH), equivalent to the instance scan of
-// Scene::intersect / Scene::occluded (scene.rs:57-140): closest hit with the
-// canonical tie rule, or any hit.
+// Ray traversal, closest or any hit, equivalent to the instance scan of
+// Scene::intersect / Scene::occluded (scene.rs:57-140) with the canonical tie
+// rule. A warp loops over a queue of n rays: the lanes take rays from the
+// queue through a shared work counter, and whenever at least `refill` lanes
+// have finished their ray (or the warp has none), the idle lanes take new rays
+// with one atomic for the warp, so the warp does not run on with a few long
+// rays. A ray's traversal does not depend on which lane or warp runs it, so
+// the results are the same as one ray per thread.
 //
-// trace_stream is a persistent loop for one warp over a queue of n rays: the
-// lanes take rays from the queue through a shared work counter, and whenever
-// at least `refill` lanes have finished their ray (or the warp has none), the
-// idle lanes take new rays with one atomic for the warp, so the warp does not
-// run on with a few long rays. A ray's traversal does not depend on which
-// lane or warp runs it, so the results are the same as one ray per thread.
+// Src supplies the rays and takes the results (kTmin / kTmax: the t range
+// that idle lanes start with; kFixedTmin: every ray's t_min is kTmin):
+//   uint32_t load(uint32_t j, TraceRay& r, int32_t& root)  ray j of the queue,
+//            the top-level root to trace; returns the id passed to store
+//   void store(uint32_t id, const TraceRay& r, TraceHit& h, bool found)
+// All 32 lanes of the warp must call it with the same n and counter.
 //
-// Each lane keeps one tagged stack:
-//   [0, 2^29)          node of an instance BVH
+// ------------------------------------------------------- binary traversal --
+// Trace node (64 B, 64-B aligned, two 256-bit loads): a GpuNode repacked by
+// k_pack_nodes at upload so that the slab tests run on packed pairs of floats
+//   q0 = (lo0.x, lo0.y)  q1 = (hi0.x, hi0.y)  q2 = (lo1.x, lo1.y)  q3 = (hi1.x, hi1.y)
+//   q4 = (lo0.z, hi0.z)  q5 = (lo1.z, hi1.z)  q6 = (ref0, ref1)    q7 = (bias, counts)
+// A child reference, which is also a stack entry:
+//   >= 0                 interior node (of an instance BVH or the top level)
+//   PYRE_REF_LEAF | s    triangles s, s + 1, ... up to the one marked last
+//   PYRE_REF_INST | k    enter instance slot k
+// A static instance whose mesh no other instance uses needs no entry: its
+// root node hangs directly below the top level (same world space), and its
+// triangle records carry its slot. `bias` gives the visiting order of two
+// children that are both hit: child 1 first iff e1 < e0 + bias. It is 0 between
+// interior children (nearest first) and +-inf where the order is fixed
+// (triangles before interior nodes, interior nodes before instance entries,
+// otherwise child 0 first). `counts` holds the leaf sizes (16 bits each).
+#define PYRE_REF_LEAF ((int)0x80000000)
+#define PYRE_REF_INST ((int)0xC0000000)
+#define PYRE_REF_SLOT 0x3fffffff
+#define PYRE_REF_LEAVE (-3)  // stack entry below an entered instance: back to world space
+#define PYRE_REF_DONE (-2)   // bottom of the stack
+#define PYRE_REF_NONE (-1)   // idle lane / no postponed leaf
+__device__ __forceinline__ bool ref_is_leaf(int r) { return r < PYRE_REF_INST; }
+__device__ __forceinline__ bool ref_is_pending(int r) { return r < PYRE_REF_DONE; }
+
+typedef unsigned long long pair32;  // two floats in one 64-bit register pair
+__device__ __forceinline__ pair32 pack2(float a, float b) {
+    pair32 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(pair32 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ pair32 add2(pair32 a, pair32 b) {
+    pair32 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ pair32 mul2(pair32 a, pair32 b) {
+    pair32 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void ldg_4x64(const void* p, pair32& a, pair32& b, pair32& c, pair32& d) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+}
+
+// The slab test of `slab`, two planes per instruction: lo - o is lo + (-o) and
+// the packed operations round like the scalar ones, so the entries and the
+// decisions are the same bits.
+__device__ __forceinline__ bool slab2(pair32 loxy, pair32 hixy, pair32 z, pair32 noxy, pair32 nozz, pair32 ixy,
+                                      pair32 izz, float tmin_ray, float tmax_cur, float* entry) {
+    float t1x, t1y, t2x, t2y, t1z, t2z;
+    unpack2(mul2(add2(loxy, noxy), ixy), t1x, t1y);
+    unpack2(mul2(add2(hixy, noxy), ixy), t2x, t2y);
+    unpack2(mul2(add2(z, nozz), izz), t1z, t2z);
+    const float tmin = fmaxf(fmaxf(fminf(t1x, t2x), fmaxf(fminf(t1y, t2y), fminf(t1z, t2z))), tmin_ray);
+    const float tmax = fminf(fminf(fmaxf(t1x, t2x), fminf(fmaxf(t1y, t2y), fmaxf(t1z, t2z))), tmax_cur);
+    *entry = tmin;
+    return tmin <= tmax;
+}
+
+// trace_binary: the warp loop over the packed binary nodes. A lane's whole state is one reference: the node it steps next,
+// the leaf or instance entry it waits with, DONE, or NONE (idle). The visiting
+// order of a ray is that of the reference's boxes and depends on nothing but
+// the ray: children nearest first, a node's leaves before its interior child,
+// and a closest-hit lane tests a leaf before its next node step (an any-hit
+// lane, whose result does not depend on the order, keeps stepping with one
+// leaf postponed).
+// What a ray needs only now and then sits in shared memory, one column per
+// thread: its world origin (leaving an instance, quad lights), direction (leaf
+// tests), time and the current hit. That leaves 10 resident blocks per SM
+// their 48 registers.
+//
+// Bound by instruction issue and load latency; against the loop it replaced
+// (scalar slab tests; leaf ranges, tags and counts in registers; every
+// instance behind an entry of its own), same bits: extend 61.4 against 81.0 ms
+// and shadow 23.5 against 30.8 ms per 1080p studio frame (125.7 against 152.7 ms
+// in all), closest hit 2.93 against 3.65 ms and any hit 0.40 against 0.50 ms on
+// the ray cases, the Cornell preset at 800x600 and 16 spp 6.82 against 8.59 ms.
+template <bool ANY, class Src>
+__device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
+                                             int refill) {
+    constexpr int LEAF_WAIT = ANY ? PYRE_LEAF_WAIT_ANY : PYRE_LEAF_WAIT_CLOSEST;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lanes_below = (1u << lane) - 1u;
+    // 64 nodes, as deep as before, plus the bottom, an instance's exit, and a
+    // leaf's sibling waiting for the leaf
+    constexpr int STACK = PYRE_STACK + 4;
+    constexpr int SK = ANY ? 8 : 0;  // bottom entries in shared memory (see trace_wide)
+    __shared__ int sstack[SK > 0 ? SK : 1][128];
+    __shared__ float sray[8][128];          // o, d, time, job
+    __shared__ int shit[ANY ? 1 : 4][128];  // u, v, instance slot, triangle slot
+    const int tid = threadIdx.x;
+    int stack[STACK - SK + 1];  // + 1: the node that waits while a postponed leaf is tested
+    int sp = 0;
+    auto spush = [&](int v) {
+        if (SK > 0 && sp < SK) sstack[sp][tid] = v;
+        else stack[sp - SK] = v;
+        ++sp;
+    };
+    auto spop = [&]() -> int {
+        --sp;
+        return (SK > 0 && sp < SK) ? sstack[sp][tid] : stack[sp - SK];
+    };
+    bool drained = false;  // warp-uniform: the queue has no rays left
+    uint32_t id = 0;
+    int node = PYRE_REF_NONE;
+    int postponed = PYRE_REF_NONE;  // any hit: a leaf met while stepping on
+    int inst = -1;                  // instance entered through an INST reference
+    float tmin = Src::kTmin, best_t = 0.0f;
+    pair32 noxy = 0, nozz = 0, ixy = 0, izz = 0;  // -origin and 1 / direction
+    bool hit_any = false;
+
+    while (true) {
+        // ---- refill idle lanes from the queue
+        if (!drained) {
+            const unsigned idle = __ballot_sync(FULL, node == PYRE_REF_NONE);
+            const int n_idle = __popc(idle);
+            if (n_idle >= refill || n_idle == 32) {
+                const int leader = __ffs(idle) - 1;
+                uint32_t base = 0;
+                if (lane == leader) base = atomicAdd(counter, (uint32_t)n_idle);
+                base = __shfl_sync(FULL, base, leader);
+                if ((uint64_t)base + (uint64_t)n_idle >= (uint64_t)n) drained = true;
+                const uint32_t j = base + (uint32_t)__popc(idle & lanes_below);
+                if (node == PYRE_REF_NONE && j < n) {
+                    int32_t root;
+                    TraceRay r;
+                    id = src.load(j, r, root);
+                    sray[0][tid] = r.o.x; sray[1][tid] = r.o.y; sray[2][tid] = r.o.z;
+                    sray[3][tid] = r.d.x; sray[4][tid] = r.d.y; sray[5][tid] = r.d.z;
+                    sray[6][tid] = r.time; sray[7][tid] = __uint_as_float(r.job);
+                    noxy = pack2(-r.o.x, -r.o.y);
+                    nozz = pack2(-r.o.z, -r.o.z);
+                    const float iz = __frcp_rn(r.d.z);
+                    ixy = pack2(__frcp_rn(r.d.x), __frcp_rn(r.d.y));
+                    izz = pack2(iz, iz);
+                    if (!Src::kFixedTmin) tmin = r.tmin;
+                    best_t = r.tmax;
+                    hit_any = false;
+                    if (!ANY) { shit[0][tid] = 0; shit[ANY ? 0 : 1][tid] = 0; shit[ANY ? 0 : 2][tid] = -1; shit[ANY ? 0 : 3][tid] = -1; }
+                    inst = -1;
+                    sp = 0;
+                    spush(PYRE_REF_DONE);
+                    node = root < 0 ? PYRE_REF_DONE : root;
+                }
+            }
+        }
+        if (!__any_sync(FULL, node != PYRE_REF_NONE)) {
+            if (drained) break;
+            continue;
+        }
+        // ---- inner phase: step nodes until at most LEAF_WAIT lanes still
+        // look for a leaf and some lane holds one
+        while (true) {
+            const bool seeks = node >= 0 && (!ANY || postponed == PYRE_REF_NONE);
+            const int seeking = __popc(__ballot_sync(FULL, seeks));
+            if (seeking == 0) break;
+            if (seeking <= LEAF_WAIT &&
+                __any_sync(FULL, ref_is_pending(node) || (ANY && postponed != PYRE_REF_NONE)))
+                break;
+#pragma unroll 1
+            for (int step = 0; step < PYRE_STEPS_PER_VOTE; ++step) {
+                if (node < 0) break;
+                const char* N = reinterpret_cast<const char*>(S.nodes) + (size_t)(uint32_t)node * 64u;
+                pair32 q0, q1, q2, q3, q4, q5, q6, q7;
+                ldg_4x64(N, q0, q1, q2, q3);
+                ldg_4x64(N + 32, q4, q5, q6, q7);
+                float e0, e1;
+                const bool h0 = slab2(q0, q1, q4, noxy, nozz, ixy, izz, tmin, best_t, &e0);
+                const bool h1 = slab2(q2, q3, q5, noxy, nozz, ixy, izz, tmin, best_t, &e1);
+                const int r0 = (int)(uint32_t)q6, r1 = (int)(uint32_t)(q6 >> 32);
+                if (h0 && h1) {
+                    const bool swap = e1 < e0 + __uint_as_float((uint32_t)q7);
+                    if (sp >= STACK) { atomicExch(S.error_flag, -5); node = PYRE_REF_DONE; break; }
+                    spush(swap ? r0 : r1);
+                    node = swap ? r1 : r0;
+                } else if (h0 || h1) {
+                    node = h0 ? r0 : r1;
+                } else {
+                    node = spop();
+                }
+                if (ANY && ref_is_leaf(node) && postponed == PYRE_REF_NONE) {
+                    postponed = node;
+                    node = spop();
+                }
+            }
+        }
+        // ---- leaf phase: the lanes that hold a leaf test its triangles
+        if (ANY && postponed != PYRE_REF_NONE) {  // the postponed leaf first; the stack has room: its entry came off it
+            spush(node);
+            node = postponed;
+            postponed = PYRE_REF_NONE;
+        }
+        if (ref_is_leaf(node)) {
+            float ox, oy, oz, oz2;
+            unpack2(noxy, ox, oy);
+            unpack2(nozz, oz, oz2);
+            const f3 o = mk3(-ox, -oy, -oz), d = mk3(sray[3][tid], sray[4][tid], sray[5][tid]);
+            do {
+                const int slot = node & PYRE_REF_SLOT;
+                const float4 A = __ldg(S.tris + 3 * (size_t)slot), B = __ldg(S.tris + 3 * (size_t)slot + 1),
+                             C = __ldg(S.tris + 3 * (size_t)slot + 2);
+                float t, u, v;
+                if (mt_test(o, d, A, B, C, &t, &u, &v) && t > tmin) {
+                    if (ANY) {
+                        if (t < best_t) { hit_any = true; node = PYRE_REF_DONE; break; }
+                    } else {
+                        const int own = __float_as_int(B.w);
+                        const int at = own >= 0 ? own : inst;
+                        bool better = t < best_t;
+                        if (!better && t == best_t && shit[ANY ? 0 : 3][tid] >= 0) {
+                            // a tie (rare): the lower Scene::primitives index, then the lower
+                            // triangle id, wins; both are read back from the records
+                            const int32_t cur = S.inst[at].orig_id, best = S.inst[shit[ANY ? 0 : 2][tid]].orig_id;
+                            const uint32_t key = __float_as_uint(A.w);
+                            const uint32_t best_key = __float_as_uint(__ldg(S.tris + 3 * (size_t)shit[ANY ? 0 : 3][tid]).w);
+                            better = cur < best || (cur == best && key < best_key);
+                        }
+                        if (better) {
+                            best_t = t;
+                            shit[0][tid] = __float_as_int(u); shit[ANY ? 0 : 1][tid] = __float_as_int(v);
+                            shit[ANY ? 0 : 2][tid] = at; shit[ANY ? 0 : 3][tid] = slot;
+                        }
+                    }
+                }
+                node = __float_as_uint(C.w) != 0u ? spop() : node + 1;
+            } while (ref_is_leaf(node));
+        }
+        // ---- instance entries (moving instances, or meshes that several
+        // instances use): the reference's root-box test at the ray's time
+        if (ref_is_pending(node) && !ref_is_leaf(node)) {
+            const f3 wo = mk3(sray[0][tid], sray[1][tid], sray[2][tid]);
+            if (node == PYRE_REF_LEAVE) {
+                noxy = pack2(-wo.x, -wo.y);
+                nozz = pack2(-wo.z, -wo.z);
+                inst = -1;
+                node = spop();
+            } else {
+                const int k = node & PYRE_REF_SLOT;
+                const DevInstance& I = S.inst[k];
+                if (sp + 2 > STACK) { atomicExch(S.error_flag, -5); node = PYRE_REF_DONE; }
+                else {
+                    if (I.more) spush(PYRE_REF_INST | (k + 1));
+                    f3 lo = wo;
+                    if (I.has_motion) {
+                        const f3 off = motion_offset(I, sray[6][tid]);
+                        if (!is_zero3(off)) lo = wo - off;
+                    }
+                    float ix, iy, iz, iz2, e;
+                    unpack2(ixy, ix, iy);
+                    unpack2(izz, iz, iz2);
+                    if (I.blas_root >= 0 && slab(I.lo[0], I.hi[0], I.lo[1], I.hi[1], I.lo[2], I.hi[2], lo,
+                                                 mk3(ix, iy, iz), tmin, best_t, &e)) {
+                        spush(PYRE_REF_LEAVE);
+                        inst = k;
+                        noxy = pack2(-lo.x, -lo.y);
+                        nozz = pack2(-lo.z, -lo.z);
+                        node = I.blas_root;
+                    } else {
+                        node = spop();
+                    }
+                }
+            }
+        }
+        // ---- finished rays hand over their result; the lane becomes idle
+        if (node == PYRE_REF_DONE) {
+            TraceRay r;
+            r.o = mk3(sray[0][tid], sray[1][tid], sray[2][tid]);
+            r.d = mk3(sray[3][tid], sray[4][tid], sray[5][tid]);
+            r.tmin = tmin;
+            r.tmax = best_t;  // read only where nothing was hit: then the ray's own
+            r.time = sray[6][tid];
+            r.job = __float_as_uint(sray[7][tid]);
+            TraceHit hit;
+            hit.t = best_t;
+            hit.light = -1;
+            hit.u = hit.v = 0.0f;
+            hit.inst = hit.tri = -1;
+            bool found = hit_any;
+            if (!ANY) {
+                hit.u = __int_as_float(shit[0][tid]); hit.v = __int_as_float(shit[ANY ? 0 : 1][tid]);
+                hit.inst = shit[ANY ? 0 : 2][tid]; hit.tri = shit[ANY ? 0 : 3][tid];
+                found = hit.tri >= 0;
+            }
+            src.store(id, r, hit, found);
+            node = PYRE_REF_NONE;
+        }
+    }
+}
+
+
+// --------------------------------------------------------- wide traversal --
+// Instance BVHs of width 4 or 8 below a binary top level. Each lane keeps one
+// tagged stack:
+//   [0, 2^28)          node of an instance BVH
+//   LEAF | n*W + k     leaf child k of wide node n
 //   TOP | n            node of the top-level BVH
 //   INST | slot        enter instance `slot` (root-box test, local origin)
 //   INST | TOP | slot  enter static instance `slot`, whose root box the
 //                      top-level step already tested
-//   LEAF | n*W + k     leaf child k of wide node n (WIDTH > 2)
 // A lane inside an instance leaves it (restores the world origin) when it
-// reaches the next TOP or INST entry: those lie below the instance's nodes.
-// With WIDTH 4 or 8 the instance BVHs are wide: a node step tests every
-// child box, continues with the nearest hit child and pushes the others
-// farthest first; leaf children are parked when they are reached.
-// Inner nodes are stepped while more than 16 lanes of the warp still need a
-// leaf (or no lane holds one); an any-hit lane that already holds one leaf
-// keeps stepping speculatively, a closest-hit lane waits for the leaf phase
-// (see STOP). Leaves found on the way are parked (at
-// most three triangle ranges, all of the current instance: a lane holding
-// leaves does not leave or enter an instance) and then tested by all lanes in
-// lock step. An any-hit lane that finds a hit is finished at the end of that
-// leaf phase.
-//
-// Src supplies the rays and takes the results (and kTmin / kTmax, the t range
-// that idle lanes start with: the range of every ray where it is fixed):
-//   uint32_t load(uint32_t j, TraceRay& r, int32_t& root)  ray j of the queue,
-//            the top-level root to trace; returns the id passed to store
-//   void store(uint32_t id, const TraceRay& r, TraceHit& h, bool found)
-// All 32 lanes of the warp must call trace_stream with the same n and counter.
+// reaches the next TOP or INST entry: those lie below the instance's nodes. A
+// node step tests every child box, continues with the nearest hit child and
+// pushes the others farthest first; leaf children are parked when they are
+// reached (an any-hit lane keeps up to three parked triangle ranges, a
+// closest-hit lane waits with its first) and tested by all lanes in lock step.
 #define PYRE_TAG_LEAF (1 << 28)
 #define PYRE_TAG_TOP (1 << 29)
 #define PYRE_TAG_INST (1 << 30)
 #define PYRE_NODE_NONE (-1)
-// top-level leaves of one static instance are entered from the top-level
-// step (INST|TOP entries); 0 keeps every instance behind an INST entry
-#ifndef PYRE_TLAS_ENTER
-#define PYRE_TLAS_ENTER 1
-#endif
-
 // Compare-exchange of (entry distance, stack entry) pairs, ascending.
 __device__ __forceinline__ void cmp_swap(float& ea, int& na, float& eb, int& nb) {
     const bool sw = eb < ea;
@@ -266,11 +540,10 @@ __device__ __forceinline__ void sort_children(float (&e)[W], int (&c)[W]) {
 }
 
 template <bool ANY, int WIDTH, class Src>
-__device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
+__device__ __forceinline__ void trace_wide(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
                                              int refill) {
-    // A lane stops stepping nodes once it holds STOP parked leaves (a binary
-    // step can park two, a wide step at most one). A closest-hit lane stops
-    // at its first: its leaves are then tested before its next node step, so
+    // A lane stops stepping nodes once it holds STOP parked leaves. A
+    // closest-hit lane stops at its first: its leaves are then tested before its next node step, so
     // the boxes it culls with its current closest distance, and its hit, do
     // not depend on the other lanes of its warp. Where two triangles are hit
     // at distances a rounding apart, a box whose rounded entry lies between
@@ -278,7 +551,8 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
     // with speculative steps that point moved with the warp, and about one
     // pixel in 10^6 of 1024^2 Cornell views changed from run to run. Any hit
     // culls with the ray's own fixed t_max, so its lanes keep stepping.
-    constexpr int STOP = ANY ? (WIDTH > 2 ? 3 : 2) : 1;
+    static_assert(WIDTH > 2, "binary BVHs are traced by trace_binary");
+    constexpr int STOP = ANY ? 3 : 1;
     constexpr int LEAF_WAIT = ANY ? PYRE_LEAF_WAIT_ANY : PYRE_LEAF_WAIT_CLOSEST;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -320,12 +594,6 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
     int node = PYRE_NODE_NONE;
     int inst = -1;
     f3 o = r.o;
-    // Parked triangle ranges: an any-hit lane keeps stepping (speculatively)
-    // while it holds at most one, so one node step never needs more than
-    // three; a closest-hit lane parks at most the two leaves of one binary
-    // step, and keeps two: fewer spills at the kernel's 56 registers (28
-    // against 34 B stored), 803.0 against 792.9 Msamples/s on the 1080p
-    // studio frame (extend 89.6 against 91.7 ms)
     constexpr int PR = ANY ? 3 : 2;
     int ls[PR], lc[PR];
 #pragma unroll
@@ -388,14 +656,7 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
                 }
                 // a top-level entry reached inside an instance: the instance's
                 // BVH is done, so the lane leaves it (once its parked leaves,
-                // which belong to the instance, are tested). Leaving without a
-                // stack entry of its own saves a node step per instance:
-                // 710.2 against 703.7 Msamples/s on the 1080p studio frame,
-                // closest hit 4.04 against 4.34 ms on the microbenchmark.
-                // Tag bits are tested once per step, and instance BVH nodes
-                // (two thirds of the steps) skip the rest: 770.9 against
-                // 767.4 Msamples/s on the 1080p studio frame. A closest-hit
-                // lane that steps holds no parked leaf (STOP is 1).
+                // which belong to the instance, are tested)
                 if (node & (PYRE_TAG_TOP | PYRE_TAG_INST)) {  // a top-level node or an instance entry
                     if (inst >= 0) {
                         if (ANY && parked) { spush(node); node = PYRE_NODE_NONE; parked = STOP; continue; }
@@ -407,7 +668,7 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
                         // tested: enter it and step its root node in this step
                         // (the lane is at the top level, so o is the world origin)
                         const int k = node & ~(PYRE_TAG_INST | PYRE_TAG_TOP);
-                        node = WIDTH > 2 ? __ldg(S.wroot + k) : __ldg(&S.inst[k].blas_root);
+                        node = __ldg(S.wroot + k);
                         if (node < 0) { node = PYRE_NODE_NONE; continue; }
                         inst = k;
                     } else if (node & PYRE_TAG_INST) {
@@ -415,7 +676,7 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
                         const int k = node & ~PYRE_TAG_INST;
                         node = PYRE_NODE_NONE;
                         const DevInstance& I = S.inst[k];
-                        const int root = WIDTH > 2 ? S.wroot[k] : I.blas_root;
+                        const int root = S.wroot[k];
                         if (root < 0) continue;
                         f3 lo = r.o;
                         if (I.has_motion) {
@@ -431,8 +692,7 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
                         continue;
                     }
                 }
-                const bool top = (node & PYRE_TAG_TOP) != 0;
-                if (WIDTH > 2 && !top) {
+                if (!(node & PYRE_TAG_TOP)) {
                     if (node & PYRE_TAG_LEAF) {  // park a leaf child of a wide node
                         const uint32_t ref = (uint32_t)(node & ~PYRE_TAG_LEAF);
                         const int32_t* NI = reinterpret_cast<const int32_t*>(S.wnodes) +
@@ -479,34 +739,24 @@ __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, 
                     continue;
                 }
                 const float4* N = S.nodes + 4 * (size_t)(node & ~PYRE_TAG_TOP);
-#if PYRE_LD256
                 float4 na, nb, nc, ndf;
                 ldg_256(N, na, nb);
                 ldg_256(N + 2, nc, ndf);
                 const int4 nd = make_int4(__float_as_int(ndf.x), __float_as_int(ndf.y), __float_as_int(ndf.z),
                                           __float_as_int(ndf.w));
-#else
-                const float4 na = __ldg(N), nb = __ldg(N + 1), nc = __ldg(N + 2);
-                const int4 nd = __ldg(reinterpret_cast<const int4*>(N + 3));
-#endif
                 float e0, e1;
                 const bool h0 = nd.x >= 0 && slab(na.x, na.y, na.z, na.w, nc.x, nc.y, o, inv, r.tmin, best_t, &e0);
                 const bool h1 = nd.y >= 0 && slab(nb.x, nb.y, nb.z, nb.w, nc.z, nc.w, o, inv, r.tmin, best_t, &e1);
                 node = PYRE_NODE_NONE;
                 const bool leaf0 = nd.z > 0, leaf1 = nd.w > 0;
-                // leaves: park triangle ranges, or queue the instances of a top-level leaf
-                if (top) {
-                    const int need = (h0 && leaf0 ? nd.z : 0) + (h1 && leaf1 ? nd.w : 0) + 1;
-                    if (sp + need > STACK) { atomicExch(S.error_flag, -5); exhausted = true; sp = 0; continue; }
-                    if (h1 && leaf1)
-                        for (int k = nd.w - 1; k >= 0; --k) spush(PYRE_TAG_INST | (nd.y + k));
-                    if (h0 && leaf0)
-                        for (int k = nd.z - 1; k >= 0; --k) spush(PYRE_TAG_INST | (nd.x + k));
-                } else {
-                    if (h0 && leaf0) { ls[parked] = nd.x; lc[parked] = nd.z; ++parked; }
-                    if (h1 && leaf1) { ls[parked] = nd.y; lc[parked] = nd.w; ++parked; }
-                }
-                const int tag = top ? PYRE_TAG_TOP : 0;
+                // a leaf queues its instances
+                const int need = (h0 && leaf0 ? nd.z : 0) + (h1 && leaf1 ? nd.w : 0) + 1;
+                if (sp + need > STACK) { atomicExch(S.error_flag, -5); exhausted = true; sp = 0; continue; }
+                if (h1 && leaf1)
+                    for (int k = nd.w - 1; k >= 0; --k) spush(PYRE_TAG_INST | (nd.y + k));
+                if (h0 && leaf0)
+                    for (int k = nd.z - 1; k >= 0; --k) spush(PYRE_TAG_INST | (nd.x + k));
+                const int tag = PYRE_TAG_TOP;
                 const bool g0 = h0 && !leaf0, g1 = h1 && !leaf1;
                 if (g0 && g1) {
                     const bool first0 = e0 <= e1;
@@ -579,6 +829,14 @@ __device__ __forceinline__ bool quad_intersect(const DevQuadLight& L, const f3& 
     *t_out = t;
     *p_out = p;
     return true;
+}
+
+// The traversal of one width (trace_binary for 2, trace_wide for 4 and 8).
+template <bool ANY, int WIDTH, class Src>
+__device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
+                                             int refill) {
+    if constexpr (WIDTH == 2) trace_binary<ANY>(S, src, n, counter, refill);
+    else trace_wide<ANY, WIDTH>(S, src, n, counter, refill);
 }
 
 // Quad lights after primitives with strict `<` (scene.rs:78-94): lights

@@ -32,10 +32,14 @@ namespace cg = cooperative_groups;
 namespace pyre {
 
 #define PYRE_MAX_DEPTH 64
-// resident blocks of 128 threads per SM for closest-hit (extend, ray queries) and any-hit (shadow) traversal
-// (with instances entered from the top-level step, 9 closest-hit blocks
-// measured 746.2 against 737.9 Msamples/s for 10 and 743.4 for 8; any hit at
-// 10 blocks took 36.0 against 34.5 ms of shadow)
+// Resident blocks of 128 threads per SM of the traversal kernels. Binary BVH,
+// 8 / 9 / 10 / 11 blocks: extend 64.0 / 61.3 / 61.3 / 64.1 ms and shadow 23.4 /
+// 23.5 / 23.3 / 24.3 ms per 1080p studio frame, 2.63 / 2.52 / 2.55 / 2.73 ms
+// and 1.20 / 1.20 / 1.17 / 1.23 ms on the Cornell preset at 800x600, closest-hit
+// queries 2.91 / 2.90 / 2.79 / 2.82 ms on the microbenchmark. 10 blocks leave
+// 48 registers, with which extend spills 12 B; 11 leave 40. Wide BVHs need
+// more registers and keep 9 blocks.
+#define PYRE_TRACE_BOUND(ANY, QUERY, WIDTH) ((WIDTH) == 2 && ((ANY) || (QUERY)) ? PYRE_TRACE_BLOCKS_10 : PYRE_TRACE_BLOCKS)
 // forward shade: threads per block and resident blocks per SM. With the
 // material-sorted queue, 224 x 4 (72 registers) measured 784.2 Msamples/s on
 // the 1080p studio frame, 192 x 5 782.9, 128 x 7 781.6 and 256 x 3 757.7.
@@ -48,8 +52,8 @@ namespace pyre {
 #ifndef PYRE_TRACE_BLOCKS
 #define PYRE_TRACE_BLOCKS 9
 #endif
-#ifndef PYRE_TRACE_BLOCKS_ANY
-#define PYRE_TRACE_BLOCKS_ANY 9
+#ifndef PYRE_TRACE_BLOCKS_10
+#define PYRE_TRACE_BLOCKS_10 10
 #endif
 #define PYRE_SORT_BINS 1024  // shade-queue sort keys: escaped, light hit, then materials
 // WaveParams::sort: how shade's queue is ordered by material
@@ -365,6 +369,7 @@ struct ExtendRays {
     // with it too, so the compiler keeps it out of registers: spills 16
     // against 28 B, 811.4 against 802.4 Msamples/s on the 1080p studio frame)
     static constexpr float kTmin = 1e-4f, kTmax = INFINITY;
+    static constexpr bool kFixedTmin = true;
     const DevScene* S;
     const PathSoA* P;
     const WaveParams* W;
@@ -394,11 +399,11 @@ struct ExtendRays {
 };
 
 // The traversal kernels are persistent grids of resident 128-thread blocks,
-// 9 per SM (56 registers). Warps wait mostly on node, triangle and stack
+// 9 or 10 per SM (56 or 48 registers). Warps wait mostly on node, triangle and stack
 // loads, so more of them per SM pay, up to where the spills that a smaller
 // register budget forces cost more than the extra warps hide.
 template <bool BATCH, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_extend(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(128, PYRE_TRACE_BOUND(false, false, WIDTH)) k_extend(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     ExtendRays<BATCH> src{&S, &P, &W, depth};
     trace_stream<false, WIDTH>(S, src, P.ctl->count[depth], &P.ctl->fetch[2 * depth], W.refill);
 }
@@ -409,6 +414,7 @@ __global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_extend(DevScene S, P
 template <bool BATCH>
 struct ShadowRays {
     static constexpr float kTmin = 1e-3f, kTmax = 0.0f;  // t_min is fixed; t_max comes with each ray
+    static constexpr bool kFixedTmin = true;
     const DevScene* S;
     const PathSoA* P;
     const WaveParams* W;
@@ -421,6 +427,7 @@ struct ShadowRays {
         r.tmin = 1e-3f;
         r.tmax = so.w;
         r.time = sd.w;
+        r.job = 0u;
         root = BATCH ? __ldcs(P->sroot + j) : S->tlas_root;
         return target;
     }
@@ -432,7 +439,7 @@ struct ShadowRays {
 };
 
 template <bool BATCH, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS_ANY) k_shadow(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(128, PYRE_TRACE_BOUND(true, false, WIDTH)) k_shadow(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     ShadowRays<BATCH> src{&S, &P, &W};
     trace_stream<true, WIDTH>(S, src, P.ctl->scount[depth], &P.ctl->fetch[2 * depth + 1], W.refill_any);
 }
@@ -990,6 +997,7 @@ __global__ void k_finalize(PathSoA P, uint32_t npix, float inv_spp, float* rad, 
 // arrays, SoA).
 struct QueryRays {
     static constexpr float kTmin = 0.0f, kTmax = 0.0f;  // both come with each ray
+    static constexpr bool kFixedTmin = false;
     const DevScene* S;
     const float* org; const float* dir; const float* tmin; const float* tmax; const float* time;
     int32_t* kind; int32_t* inst; int32_t* tri; float* tt; float* uu; float* vv; uint8_t* occluded;
@@ -999,6 +1007,7 @@ struct QueryRays {
         r.tmin = tmin[i];
         r.tmax = tmax[i];
         r.time = time ? time[i] : 0.0f;
+        r.job = 0u;
         root = S->tlas_root;
         return i;
     }
@@ -1021,7 +1030,7 @@ struct QueryRays {
 };
 
 template <bool ANY, int WIDTH>
-__global__ void __launch_bounds__(128, ANY ? PYRE_TRACE_BLOCKS_ANY : PYRE_TRACE_BLOCKS) k_intersect(DevScene S, QueryRays q, uint32_t n, unsigned int* counter,
+__global__ void __launch_bounds__(128, PYRE_TRACE_BOUND(ANY, true, WIDTH)) k_intersect(DevScene S, QueryRays q, uint32_t n, unsigned int* counter,
                                                    int refill) {
     QueryRays src = q;
     src.S = &S;
@@ -1521,6 +1530,8 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
     DevScene D;
     int rc = select_bvh(ctx, const_cast<pyre_scene*>(scene), params ? params->bvh_width : 0u, &D, &W.bvh_width);
     if (rc) return rc;
+    if (W.bvh_width > 2)
+        for (uint32_t j = 0; j < n_jobs; ++j) dj[j].tlas_root = scene->top_root(jobs[j].part);
     const uint32_t ns = std::max(W.ns, 1u);
 
     // ---- workspace: path state, accumulators, tables, staging film

@@ -20,12 +20,19 @@ struct pyre_scene {
     std::vector<int32_t> part_tlas;    // host copies of the per-part tables
     std::vector<uint32_t> part_light;  // (first, count) per part
     uint64_t device_bytes = 0;
-    // wide BVHs built on first use (index 0: width 4, 1: width 8)
+    // wide BVHs built on first use (index 0: width 4, 1: width 8), and the top
+    // level they hang below: GpuNodes with instance entries, from node
+    // top_base of the binary BVH on (host copy; on the device once a wide BVH
+    // is built, with node indices from 0)
     struct Wide {
         float4* nodes = nullptr;
         int32_t* root = nullptr;  // per instance slot
         uint64_t n_nodes = 0;
     } wide[2];
+    std::vector<pyre::GpuNode> top;
+    int32_t top_base = 0;
+    pyre::GpuNode* d_top = nullptr;
+    int32_t top_root(uint32_t part) const { return part_tlas[part] < 0 ? -1 : part_tlas[part] - top_base; }
     int bvh_width = 2;  // traversal width when a call does not choose one
 };
 
