@@ -303,19 +303,22 @@ __global__ void k_pack_nodes(GpuNode* __restrict__ nodes, uint32_t n_nodes, uint
         f[12] = __int_as_float(ref[0]); f[13] = __int_as_float(ref[1]);
         f[14] = bias; f[15] = __uint_as_float(counts);
         float4* w = reinterpret_cast<float4*>(nodes + i);
-        for (int q = 0; q < 4; ++q) w[q] = out[q];
+        for (uint32_t q = 0; q < 4; ++q) w[q ^ PYRE_NODE_SWAP(i)] = out[q];
     }
 }
 
 // A trace node of an instance BVH back as the GpuNode it was packed from.
-GpuNode unpack_node(const GpuNode& packed) {
+GpuNode unpack_node(const GpuNode& packed, uint32_t index) {
     float f[16];
-    std::memcpy(f, &packed, sizeof f);
+    int32_t d[16];
+    for (uint32_t q = 0; q < 4; ++q) {
+        std::memcpy(f + 4 * q, reinterpret_cast<const char*>(&packed) + 16 * (q ^ PYRE_NODE_SWAP(index)), 16);
+        std::memcpy(d + 4 * q, f + 4 * q, 16);
+    }
     GpuNode g;
-    uint32_t counts;
-    std::memcpy(&counts, &packed.d[3], 4);
+    const uint32_t counts = (uint32_t)d[15];
     for (int s = 0; s < 2; ++s) {
-        const int32_t ref = packed.d[s];
+        const int32_t ref = d[12 + s];
         Aabb b;
         b.lo = mk3(f[4 * s], f[4 * s + 1], f[8 + 2 * s]);
         b.hi = mk3(f[4 * s + 2], f[4 * s + 3], f[9 + 2 * s]);
@@ -832,7 +835,7 @@ int select_bvh(pyre_ctx* ctx, pyre_scene* scene, uint32_t requested, DevScene* d
                                       cudaMemcpyDeviceToHost));
         PYRE_CUDA_TRY(ctx, cudaMemcpy(inst.data(), scene->dev.inst, inst.size() * sizeof(DevInstance),
                                       cudaMemcpyDeviceToHost));
-        for (GpuNode& g : bin) g = unpack_node(g);
+        for (size_t k = 0; k < bin.size(); ++k) bin[k] = unpack_node(bin[k], (uint32_t)k);
         std::vector<float> flat;
         std::map<int32_t, int32_t> wide_of;
         std::vector<int32_t> roots(inst.size(), -1);

@@ -249,6 +249,20 @@ __device__ __forceinline__ void ldg_4x64(const void* p, pair32& a, pair32& b, pa
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
 }
 
+// The address of q0..q3 of trace node n; q4..q7 sit at that address ^ 32. Nodes
+// with bit 1 of their index set hold their halves swapped: otherwise the lanes
+// of a warp, each at its own node, would all read offset 0 or 64 of a 128-B
+// line with one load and 32 or 96 with the other, half of the L1's banks at a
+// time. L1 data cycles bound the traversal once its instructions were halved:
+// extend 55.6 against 58.2 ms and shadow 21.4 against 23.1 ms per 1080p studio
+// frame, closest-hit queries 2.54 against 2.62 ms. (Random 64-B fetches by 32
+// lanes from an L1-resident array: 35.6 against 46.4 cycles; four 128-bit loads
+// 77.3.)
+#define PYRE_NODE_SWAP(n) ((n) & 2u)
+__device__ __forceinline__ uint64_t trace_node_half(const float4* nodes, uint32_t n) {
+    return reinterpret_cast<uint64_t>(nodes) + ((uint64_t)n * 64u | (PYRE_NODE_SWAP(n) << 4));
+}
+
 // The slab test of `slab`, two planes per instruction: lo - o is lo + (-o) and
 // the packed operations round like the scalar ones, so the entries and the
 // decisions are the same bits.
@@ -282,6 +296,24 @@ __device__ __forceinline__ bool slab2(pair32 loxy, pair32 hixy, pair32 z, pair32
 // and shadow 23.5 against 30.8 ms per 1080p studio frame (125.7 against 152.7 ms
 // in all), closest hit 2.93 against 3.65 ms and any hit 0.40 against 0.50 ms on
 // the ray cases, the Cornell preset at 800x600 and 16 spp 6.82 against 8.59 ms.
+// A warp that needs rays takes a share of the queue: consecutive rays, which
+// start close together, so that what one ray brought into L1 serves the next.
+// A share is at most PYRE_SHARE rays and a 64th of what a warp gets on average,
+// whole warps of it; below that a warp takes what its idle lanes need, and the
+// last rays of the queue stay spread over all warps. On the 1080p studio frame
+// (133 M camera rays) 118.6 ms against 119.8 without shares; the Cornell preset
+// at 800x600 (7.7 M camera rays) 6.10 with a 32nd, 6.05 with a 64th, 6.04 without.
+#ifndef PYRE_SHARE
+#define PYRE_SHARE 128
+#endif
+// Bottom entries of a lane's stack kept in shared memory (entry-major, so a
+// lane always uses its own bank), the rest in local memory, whose lines the
+// nodes push out of L1 (26 % of the stack loads hit): 0 / 4 / 8 / 12 / 16
+// entries gave 62.4 / 61.6 / 60.0 / 59.8 / 59.8 ms of extend per 1080p studio
+// frame and 2.82 / 2.76 / 2.63 / 2.62 / 2.63 ms of closest-hit queries.
+#ifndef PYRE_STACK_SHARED
+#define PYRE_STACK_SHARED 12
+#endif
 template <bool ANY, class Src>
 __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
                                              int refill) {
@@ -292,23 +324,25 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
     // 64 nodes, as deep as before, plus the bottom, an instance's exit, and a
     // leaf's sibling waiting for the leaf
     constexpr int STACK = PYRE_STACK + 4;
-    constexpr int SK = ANY ? 8 : 0;  // bottom entries in shared memory (see trace_wide)
-    __shared__ int sstack[SK > 0 ? SK : 1][128];
+    constexpr int SK = PYRE_STACK_SHARED;
+    __shared__ int sstack[SK][128];  // blocks have at most 128 threads
     __shared__ float sray[8][128];          // o, d, time, job
     __shared__ int shit[ANY ? 1 : 4][128];  // u, v, instance slot, triangle slot
     const int tid = threadIdx.x;
     int stack[STACK - SK + 1];  // + 1: the node that waits while a postponed leaf is tested
     int sp = 0;
     auto spush = [&](int v) {
-        if (SK > 0 && sp < SK) sstack[sp][tid] = v;
+        if (sp < SK) sstack[sp][tid] = v;
         else stack[sp - SK] = v;
         ++sp;
     };
     auto spop = [&]() -> int {
         --sp;
-        return (SK > 0 && sp < SK) ? sstack[sp][tid] : stack[sp - SK];
+        return sp < SK ? sstack[sp][tid] : stack[sp - SK];
     };
     bool drained = false;  // warp-uniform: the queue has no rays left
+    uint32_t next = 0, end = 0;  // warp-uniform: the rest of the warp's share of the queue
+    const uint32_t share = min((uint32_t)PYRE_SHARE, n / (gridDim.x * (blockDim.x >> 5) * 64u) & ~31u);
     uint32_t id = 0;
     int node = PYRE_REF_NONE;
     int postponed = PYRE_REF_NONE;  // any hit: a leaf met while stepping on
@@ -319,17 +353,25 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
 
     while (true) {
         // ---- refill idle lanes from the queue
-        if (!drained) {
+        if (!drained || next < end) {
             const unsigned idle = __ballot_sync(FULL, node == PYRE_REF_NONE);
             const int n_idle = __popc(idle);
             if (n_idle >= refill || n_idle == 32) {
-                const int leader = __ffs(idle) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(counter, (uint32_t)n_idle);
-                base = __shfl_sync(FULL, base, leader);
-                if ((uint64_t)base + (uint64_t)n_idle >= (uint64_t)n) drained = true;
-                const uint32_t j = base + (uint32_t)__popc(idle & lanes_below);
-                if (node == PYRE_REF_NONE && j < n) {
+                const uint32_t avail = end - next, rank = (uint32_t)__popc(idle & lanes_below);
+                uint32_t j = next + rank, stop = end;
+                next += min((uint32_t)n_idle, avail);
+                if ((uint32_t)n_idle > avail && !drained) {  // the rest of the idle lanes start the warp's next share
+                    const uint32_t need = (uint32_t)n_idle - avail, take = max(share, need);
+                    uint32_t base = 0;
+                    if (lane == 0) base = atomicAdd(counter, take);
+                    base = __shfl_sync(FULL, base, 0);
+                    if ((uint64_t)base + take >= (uint64_t)n) drained = true;
+                    base = min(base, n);
+                    end = min(base + take, n);
+                    if (rank >= avail) { j = base + (rank - avail); stop = end; }
+                    next = min(base + need, end);
+                }
+                if (node == PYRE_REF_NONE && j < stop) {
                     int32_t root;
                     TraceRay r;
                     id = src.load(j, r, root);
@@ -353,7 +395,7 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
             }
         }
         if (!__any_sync(FULL, node != PYRE_REF_NONE)) {
-            if (drained) break;
+            if (drained && next == end) break;
             continue;
         }
         // ---- inner phase: step nodes until at most LEAF_WAIT lanes still
@@ -368,10 +410,10 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
 #pragma unroll 1
             for (int step = 0; step < PYRE_STEPS_PER_VOTE; ++step) {
                 if (node < 0) break;
-                const char* N = reinterpret_cast<const char*>(S.nodes) + (size_t)(uint32_t)node * 64u;
+                const uint64_t N = trace_node_half(S.nodes, (uint32_t)node);
                 pair32 q0, q1, q2, q3, q4, q5, q6, q7;
-                ldg_4x64(N, q0, q1, q2, q3);
-                ldg_4x64(N + 32, q4, q5, q6, q7);
+                ldg_4x64(reinterpret_cast<const void*>(N), q0, q1, q2, q3);
+                ldg_4x64(reinterpret_cast<const void*>(N ^ 32u), q4, q5, q6, q7);
                 float e0, e1;
                 const bool h0 = slab2(q0, q1, q4, noxy, nozz, ixy, izz, tmin, best_t, &e0);
                 const bool h1 = slab2(q2, q3, q5, noxy, nozz, ixy, izz, tmin, best_t, &e1);

@@ -33,13 +33,12 @@ namespace pyre {
 
 #define PYRE_MAX_DEPTH 64
 // Resident blocks of 128 threads per SM of the traversal kernels. Binary BVH,
-// 8 / 9 / 10 / 11 blocks: extend 64.0 / 61.3 / 61.3 / 64.1 ms and shadow 23.4 /
-// 23.5 / 23.3 / 24.3 ms per 1080p studio frame, 2.63 / 2.52 / 2.55 / 2.73 ms
-// and 1.20 / 1.20 / 1.17 / 1.23 ms on the Cornell preset at 800x600, closest-hit
-// queries 2.91 / 2.90 / 2.79 / 2.82 ms on the microbenchmark. 10 blocks leave
-// 48 registers, with which extend spills 12 B; 11 leave 40. Wide BVHs need
-// more registers and keep 9 blocks.
-#define PYRE_TRACE_BOUND(ANY, QUERY, WIDTH) ((WIDTH) == 2 && ((ANY) || (QUERY)) ? PYRE_TRACE_BLOCKS_10 : PYRE_TRACE_BLOCKS)
+// 8 / 9 / 10 blocks: extend 56.9 / 55.5 / 62 ms (10 leave 48 registers, with
+// spills) and shadow 21.7 / 21.7 / 21.4 ms per 1080p studio frame, 1.16 / 1.16 /
+// 1.12 ms on the Cornell preset at 800x600, closest-hit queries 2.68 / 2.53 /
+// 2.56 ms, any hit 0.344 / 0.344 / 0.356 ms. Wide BVHs need more registers.
+#define PYRE_TRACE_BLOCKS 9
+#define PYRE_SHADOW_BLOCKS(WIDTH) ((WIDTH) == 2 ? 10 : 9)
 // forward shade: threads per block and resident blocks per SM. With the
 // material-sorted queue, 224 x 4 (72 registers) measured 784.2 Msamples/s on
 // the 1080p studio frame, 192 x 5 782.9, 128 x 7 781.6 and 256 x 3 757.7.
@@ -48,12 +47,6 @@ namespace pyre {
 #endif
 #ifndef PYRE_SHADE_BLOCKS
 #define PYRE_SHADE_BLOCKS 4
-#endif
-#ifndef PYRE_TRACE_BLOCKS
-#define PYRE_TRACE_BLOCKS 9
-#endif
-#ifndef PYRE_TRACE_BLOCKS_10
-#define PYRE_TRACE_BLOCKS_10 10
 #endif
 #define PYRE_SORT_BINS 1024  // shade-queue sort keys: escaped, light hit, then materials
 // WaveParams::sort: how shade's queue is ordered by material
@@ -403,7 +396,7 @@ struct ExtendRays {
 // loads, so more of them per SM pay, up to where the spills that a smaller
 // register budget forces cost more than the extra warps hide.
 template <bool BATCH, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BOUND(false, false, WIDTH)) k_extend(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_extend(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     ExtendRays<BATCH> src{&S, &P, &W, depth};
     trace_stream<false, WIDTH>(S, src, P.ctl->count[depth], &P.ctl->fetch[2 * depth], W.refill);
 }
@@ -439,7 +432,7 @@ struct ShadowRays {
 };
 
 template <bool BATCH, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BOUND(true, false, WIDTH)) k_shadow(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(128, PYRE_SHADOW_BLOCKS(WIDTH)) k_shadow(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     ShadowRays<BATCH> src{&S, &P, &W};
     trace_stream<true, WIDTH>(S, src, P.ctl->scount[depth], &P.ctl->fetch[2 * depth + 1], W.refill_any);
 }
@@ -1030,7 +1023,7 @@ struct QueryRays {
 };
 
 template <bool ANY, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BOUND(ANY, true, WIDTH)) k_intersect(DevScene S, QueryRays q, uint32_t n, unsigned int* counter,
+__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_intersect(DevScene S, QueryRays q, uint32_t n, unsigned int* counter,
                                                    int refill) {
     QueryRays src = q;
     src.S = &S;
