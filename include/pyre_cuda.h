@@ -263,9 +263,10 @@ typedef struct pyre_render_params {
     uint32_t env_sampling;           /* PYRE_ENV_ALIAS or PYRE_ENV_CDF */
     uint32_t wave_paths;             /* paths in flight per wave; 0 = automatic (what a quarter
                                         of the free device memory holds, 8 Mi to 128 Mi) */
-    uint32_t block_size;             /* threads per block of the stage kernels (at most 224
-                                        for the forward shade, 128 for the traversals);
-                                        0 = 256 / 224 / 128 */
+    uint32_t block_size;             /* threads per block of the stage kernels (at most 256;
+                                        224 for the forward shade of a scene with an
+                                        environment, 128 for the traversals);
+                                        0 = those */
     uint32_t sort_by_material;       /* order the shade queue by material: 1 = within
                                         tiles of 4096 entries, 2 = off, 3 = the whole
                                         queue, 0 = the default (off; 3 in pyre_backward) */

@@ -2,8 +2,8 @@
 
 Knobs (pyre_render_params): wave_paths (queue capacity = paths in flight per
 wave), block_size (threads per block of the stage kernels, capped at 224 for
-the forward shade and 128 for the traversals; 0 = the library's defaults
-256 / 224 / 128), use_graph (CUDA-graph replay),
+the forward shade of a scene with an environment and at 128 for the
+traversals; 0 = those, 256 elsewhere), use_graph (CUDA-graph replay),
 sort_by_material (shade visits the live paths sorted by material) and
 refill_lanes (a warp refetches rays once this many of its lanes are idle) and
 bvh_width (instance BVHs traversed as binary, 4-wide or 8-wide nodes).

@@ -108,8 +108,8 @@ __device__ __forceinline__ void env_texel_weights(const DevEnv& E, f2 uv, uint32
     float fy = clampf_(v * (float)h - 0.5f, 0.0f, (float)h - 1.0f);
     int32_t x0i = sat_i32(floorf(fx)), y0i = sat_i32(floorf(fy));
     float dx = fx - (float)x0i, dy = fy - (float)y0i;
-    int32_t x0 = ((x0i % w) + w) % w;
-    int32_t x1 = ((x0 + 1) % w + w) % w;
+    int32_t x0 = env_wrap(x0i, w);
+    int32_t x1 = env_wrap(x0 + 1, w);
     int32_t y0 = min(max(y0i, 0), h - 1);
     int32_t y1 = min(y0 + 1, h - 1);
     idx[0] = (uint32_t)(y0 * w + x0); wt[0] = (1.0f - dx) * (1.0f - dy);

@@ -667,12 +667,7 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
 
     // ---- materials and lights
     std::vector<DevMaterial> mats(desc->n_materials);
-    for (uint32_t i = 0; i < desc->n_materials; ++i) {
-        const pyre_material_desc& m = desc->materials[i];
-        DevMaterial& d = mats[i];
-        for (int c = 0; c < 3; ++c) d.base[c] = m.base_color[c];
-        d.kind = m.kind; d.metallic = m.metallic; d.roughness = m.roughness; d.specular = m.specular; d.pad = 0;
-    }
+    for (uint32_t i = 0; i < desc->n_materials; ++i) mats[i] = make_material(desc->materials[i]);
     std::vector<DevQuadLight> lights(desc->n_lights);
     for (uint32_t i = 0; i < desc->n_lights; ++i) {  // DiffuseAreaQuadLight::new, light.rs:61-76
         const pyre_quad_light_desc& l = desc->lights[i];
@@ -922,10 +917,7 @@ int pyre_scene_set_materials(pyre_ctx* ctx, pyre_scene* scene, const pyre_materi
     std::vector<DevMaterial> mats(n);
     for (uint32_t i = 0; i < n; ++i) {
         if (materials[i].kind > PYRE_MAT_DISNEY) return set_error(ctx, PYRE_ERR_INVALID, "unknown material kind");
-        DevMaterial& d = mats[i];
-        for (int c = 0; c < 3; ++c) d.base[c] = materials[i].base_color[c];
-        d.kind = materials[i].kind; d.metallic = materials[i].metallic; d.roughness = materials[i].roughness;
-        d.specular = materials[i].specular; d.pad = 0;
+        mats[i] = make_material(materials[i]);
     }
     cudaSetDevice(ctx->device);
     PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1038,10 +1030,7 @@ int pyre_bsdf_query(pyre_ctx* ctx, const pyre_material_desc* mat, uint32_t n, co
     cudaStream_t st = ctx->stream;
     PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(b, wo, (size_t)n * 12, cudaMemcpyHostToDevice, st));
     PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(b + b_wo, u, (size_t)n * 8, cudaMemcpyHostToDevice, st));
-    Bsdf bs;
-    bs.kind = mat->kind;
-    bs.base = mk3(mat->base_color[0], mat->base_color[1], mat->base_color[2]);
-    bs.metallic = mat->metallic; bs.roughness = mat->roughness; bs.specular = mat->specular;
+    const Bsdf bs = make_bsdf(make_material(*mat));
     k_bsdf_query<<<(n + 255) / 256, 256, 0, st>>>(bs, (const float*)b, (const float*)(b + b_wo), n,
                                                    (float*)(b + b_wo + b_u));
     PYRE_CUDA_TRY(ctx, cudaGetLastError());

@@ -39,10 +39,16 @@ struct alignas(16) DevInstance {
     uint32_t direct;       // static, and no other instance uses its mesh: its root hangs below the top level
 };
 
-struct alignas(16) DevMaterial {
+// A material and what the BSDF derives from it alone (make_material), 64 B.
+struct alignas(64) DevMaterial {
     float base[3];
     uint32_t kind;
-    float metallic, roughness, specular, pad;
+    float metallic, roughness, specular;
+    float alpha;   // GGX alpha
+    float kd[3];   // base (1 - metallic) / pi; Lambertian: albedo / pi
+    float pd;      // probability of the diffuse lobe
+    float f0[3];   // specular reflectance at normal incidence
+    float ps;      // probability of the specular lobe
 };
 
 struct DevQuadLight {

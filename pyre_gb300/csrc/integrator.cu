@@ -22,6 +22,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "internal.h"
 #include "adjoint.cuh"
@@ -39,15 +40,6 @@ namespace pyre {
 // 2.56 ms, any hit 0.344 / 0.344 / 0.356 ms. Wide BVHs need more registers.
 #define PYRE_TRACE_BLOCKS 9
 #define PYRE_SHADOW_BLOCKS(WIDTH) ((WIDTH) == 2 ? 10 : 9)
-// forward shade: threads per block and resident blocks per SM. With the
-// material-sorted queue, 224 x 4 (72 registers) measured 784.2 Msamples/s on
-// the 1080p studio frame, 192 x 5 782.9, 128 x 7 781.6 and 256 x 3 757.7.
-#ifndef PYRE_SHADE_THREADS
-#define PYRE_SHADE_THREADS 224
-#endif
-#ifndef PYRE_SHADE_BLOCKS
-#define PYRE_SHADE_BLOCKS 4
-#endif
 #define PYRE_SORT_BINS 1024  // shade-queue sort keys: escaped, light hit, then materials
 // WaveParams::sort: how shade's queue is ordered by material
 #define PYRE_SORT_OFF 0
@@ -602,13 +594,25 @@ __global__ void __launch_bounds__(256) k_sort_tile(DevScene S, PathSoA P, uint32
 // One path vertex of PathIntegrator::integrate (integrator.rs:242-388).
 // ADJ: the path-replay adjoint of the same vertex (pyre_backward): the same
 // draws and decisions, plus the derivatives of its terms.
-// Forward shade: 4 resident blocks of 224 threads (72 registers); it is
-// latency-bound, and 28 warps per SM beat 24 (3 blocks of 256, 80
-// registers) by 0.3 % on the 1080p studio frame. The adjoint variant keeps
-// 3 blocks of 256: at 72 registers its spills would grow.
-template <bool BATCH, bool ADJ = false>
-__global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE_SHADE_BLOCKS) k_shade(DevScene S, PathSoA P, WaveParams W,
-                                                                        uint32_t depth) {
+// LIGHTS: the kinds of light the scene has (SHADE_QUADS, SHADE_ENV); without an
+// environment its code is left out, which a kernel this large pays for in
+// registers and instruction fetches: 2.05 against 2.19 ms of shade on the Cornell
+// preset at 800x600 and 16 spp, 213 against 215 ms on a batch of 40 views.
+// Threads and resident blocks: bound by load latency, 24 to 28 warps per SM.
+// Quad lights only: 256 x 3 (80 registers), 128 x 6 / 192 x 4 the same, 224 x 4
+// 2.19 against 2.05 ms and 236 against 213 ms on the batch. With an environment:
+// 224 x 4 (72 registers) 35.6 ms per 1080p studio frame, 256 x 3 36.6, 192 x 5 and
+// 128 x 8 37.9 and 42.5 (before the material terms below). The adjoint keeps 3
+// blocks of 256; leaving out the quad lights there gave 14.9 against 15.2 ms of
+// backward on the 512^2 problem (the forward lost 1 ms of 35.6 that way).
+#define SHADE_QUADS 1
+#define SHADE_ENV 2
+constexpr int shade_threads(int lights) { return lights == SHADE_QUADS ? 256 : 224; }
+constexpr int shade_blocks(int lights) { return lights == SHADE_QUADS ? 3 : 4; }
+template <bool BATCH, bool ADJ, int LIGHTS>
+__global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : shade_blocks(LIGHTS))
+    k_shade(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+    constexpr bool QUADS = (LIGHTS & SHADE_QUADS) != 0, ENV = (LIGHTS & SHADE_ENV) != 0;
     GradSmem G{nullptr, nullptr, nullptr};
     if (ADJ) G = grad_smem_begin(W.env_cache != 0, W.smem_grad != 0, W.n_mat);
     const uint32_t n = P.ctl->count[depth];
@@ -686,7 +690,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE
                          make_float4(0.0f, 0.0f, 0.0f, 0.0f));
             }
             // Escaped: environment radiance with MIS against the BSDF arm (integrator.rs:243-259).
-            if (S.has_env) {
+            if (ENV && S.has_env) {
                 const f2 uv = env_dir_to_uv(ray_d);
                 f3 le = env_texture(S.env, uv) * S.env.intensity;
                 if (!is_zero3(le)) {
@@ -702,7 +706,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE
                     if (ADJ) scatter_env(S.env, W.env_grad, G, uv, delta * beta * w_adj);
                 }
             }
-        } else if (code <= -2) {
+        } else if (QUADS && code <= -2) {
             // Quad light hit (integrator.rs:262-295).
             const DevQuadLight& Lt = S.lights[-2 - code];
             if (depth == 0) {
@@ -749,7 +753,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE
             if (wo.z > 0.0f) {
                 Rng g = load_rng(P.rng, i);
                 const f3 p_off = p + 1e-3f * ns;
-                uint32_t lfirst = 0, lcount = S.n_lights;
+                uint32_t lfirst = 0, lcount = QUADS ? S.n_lights : 0u;
                 if (BATCH) {
                     lfirst = JB->light_first; lcount = JB->light_count;
                 }
@@ -758,16 +762,17 @@ __global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE
                 // (integrator.rs:307-333), NEE for the environment (335-354),
                 // then the BSDF sample (356-387). All three evaluate the BSDF
                 // at one call site, so the kernel holds one copy of it.
-                const uint32_t n_nee = lcount + (S.has_env ? 1u : 0u);
+                const uint32_t n_nee = lcount + (ENV && S.has_env ? 1u : 0u);
                 for (uint32_t s = 0; s <= n_nee; ++s) {
                     const f2 u2 = g.next_vec2();
-                    const bool bsdf_arm = s == n_nee, env_arm = !bsdf_arm && s == lcount;
+                    const bool bsdf_arm = s == n_nee, env_arm = ENV && !bsdf_arm && (!QUADS || s == lcount);
                     f3 wi, wi_w = splat3(0.0f), le = splat3(0.0f), sh_dir = splat3(0.0f);
                     float lpdf = 0.0f, sh_tmax = INF;
                     bool sh_ray = true;
+                    wi = splat3(0.0f);
                     if (bsdf_arm) {
                         if (!bsdf_sample_dir(mat, wo, u2, &wi)) break;
-                    } else if (!env_arm) {
+                    } else if (QUADS && !env_arm) {
                         const DevQuadLight& Lt = S.lights[lfirst + s];
                         f3 lpos;
                         if (!quad_sample(Lt, p, u2, &lpos, &wi_w, &lpdf)) continue;
@@ -781,7 +786,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE
                         sh_ray = dist > 0.0f;
                         sh_dir = tf / dist;
                         sh_tmax = dist - 1e-3f;
-                    } else {
+                    } else if (ENV) {
                         env_sample(S.env, u2, W.env_cdf, &wi_w, &le, &lpdf);
                         if (!(lpdf > 0.0f) || is_zero3(le)) continue;
                         wi = to_local(fr, wi_w);
@@ -827,7 +832,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : PYRE_SHADE_THREADS, ADJ ? 3 : PYRE
                     if (is_zero3(f)) continue;
                     const float w = power_heuristic(lpdf, pdf_b);
                     const f3 contrib = beta * f * le * wi.z * w / lpdf;
-                    const size_t sidx = (size_t)i * W.ns + (env_arm ? S.n_lights : s);
+                    const size_t sidx = (size_t)i * W.ns + (!QUADS ? 0u : (env_arm ? S.n_lights : s));
                     __stcs(&P.pend[sidx], make_float4(contrib.x, contrib.y, contrib.z, 1.0f));
                     if (ADJ) {  // park the slot's d/d params (and texels); cleared if occluded
                         float4* G = P.gpend + PYRE_GSLOT * sidx;
@@ -1105,26 +1110,41 @@ uint64_t default_wave_paths(pyre_ctx* ctx, uint32_t ns, bool batch, bool adjoint
 
 struct Launch {
     int block_stage = 256;  // raygen, accumulate, adjoint shade (at most 256)
-    int block_shade = PYRE_SHADE_THREADS;  // forward shade (at most PYRE_SHADE_THREADS)
+    int block_shade = 0;    // forward shade (at most shade_threads of the scene's lights)
+    int lights = SHADE_QUADS;  // the forward shade's LIGHTS
     int block_trace = 128;  // extend, shadow (at most 128)
     int grid_raygen, grid_shade, grid_extend, grid_shadow, grid_acc, grid_sort;
 };
 
+// The LIGHTS of a scene's shade kernels, and f called with them as a compile-time constant (batches carry no environment).
+int scene_lights(const DevScene& S) {
+    const int l = (S.n_lights ? SHADE_QUADS : 0) | (S.has_env ? SHADE_ENV : 0);
+    return l ? l : SHADE_QUADS;
+}
+template <bool BATCH, class F>
+void with_lights(int lights, F f) {
+    if constexpr (!BATCH) {
+        if (lights != SHADE_QUADS) return f(std::integral_constant<int, SHADE_QUADS | SHADE_ENV>());
+    }
+    f(std::integral_constant<int, SHADE_QUADS>());
+}
+
 // Grid sizes for the stage kernels: persistent grids of resident blocks.
-// block_size (0 = defaults: 256 for raygen and accumulate, 224 for the
-// forward shade, 128 for the traces) sets them all, capped at 224 for the
-// forward shade and 128 for the traces.
+// block_size (0 = defaults: 256 for raygen and accumulate, shade_threads for
+// the forward shade, 128 for the traces) sets them all, capped at those.
 template <bool BATCH>
-Launch make_launch(pyre_ctx* ctx, uint32_t block_size, int width) {
+Launch make_launch(pyre_ctx* ctx, const DevScene& S, uint32_t block_size, int width) {
     Launch L;
+    L.lights = scene_lights(S);
+    L.block_shade = shade_threads(L.lights);
     if (block_size) {
         const int b = (int)std::max(32u, std::min(256u, block_size / 32 * 32));
         L.block_stage = b;
-        L.block_shade = std::min(b, PYRE_SHADE_THREADS);
+        L.block_shade = std::min(b, L.block_shade);
         L.block_trace = std::min(b, 128);
     }
     L.grid_raygen = grid_for(ctx, k_raygen<BATCH>, L.block_stage);
-    L.grid_shade = grid_for(ctx, k_shade<BATCH>, L.block_shade);
+    with_lights<BATCH>(L.lights, [&](auto l) { L.grid_shade = grid_for(ctx, k_shade<BATCH, false, l()>, L.block_shade); });
     L.grid_extend = width == 8 ? grid_for(ctx, k_extend<BATCH, 8>, L.block_trace)
                     : width == 4 ? grid_for(ctx, k_extend<BATCH, 4>, L.block_trace)
                                  : grid_for(ctx, k_extend<BATCH, 2>, L.block_trace);
@@ -1192,7 +1212,7 @@ void enqueue_wave(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const Wave
         launch_extend<false>(st, Lc, S, P, W, d);
         mark(ctx, STAGE_SHADE);
         if (W.sort) enqueue_sort(ctx, S, P, Lc, d, W.sort);
-        k_shade<false><<<Lc.grid_shade, Lc.block_shade, 0, st>>>(S, P, W, d);
+        with_lights<false>(Lc.lights, [&](auto l) { k_shade<false, false, l()><<<Lc.grid_shade, Lc.block_shade, 0, st>>>(S, P, W, d); });
         if (W.ns > 0) {
             mark(ctx, STAGE_SHADOW);
             launch_shadow<false>(st, Lc, S, P, W, d);
@@ -1216,7 +1236,7 @@ void enqueue_wave_batch(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, cons
         launch_extend<true>(st, Lc, S, P, W, d);
         mark(ctx, STAGE_SHADE);
         if (W.sort) enqueue_sort(ctx, S, P, Lc, d, W.sort);
-        k_shade<true><<<Lc.grid_shade, Lc.block_shade, 0, st>>>(S, P, W, d);
+        k_shade<true, false, SHADE_QUADS><<<Lc.grid_shade, Lc.block_shade, 0, st>>>(S, P, W, d);
         if (W.ns > 0) {
             mark(ctx, STAGE_SHADOW);
             launch_shadow<true>(st, Lc, S, P, W, d);
@@ -1353,7 +1373,7 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
     S.keep_L = keep;
     if (film->mem == PYRE_MEM_HOST && (rc = ensure_workspace(ctx, ctx->io_ws, film_bytes))) return rc;
 
-    const Launch Lc = make_launch<false>(ctx, rp.block_size, W.bvh_width);
+    const Launch Lc = make_launch<false>(ctx, D, rp.block_size, W.bvh_width);
 
     cudaStream_t st = ctx->stream;
     PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_r, 0, (size_t)W.npix * sizeof(float4), st));
@@ -1554,7 +1574,7 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
     PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_n, 0, total_pix * sizeof(float4), st));
     PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.ctl, 0, sizeof(WaveCtl), st));
 
-    const Launch Lc = make_launch<true>(ctx, params ? params->block_size : 0u, W.bvh_width);
+    const Launch Lc = make_launch<true>(ctx, D, params ? params->block_size : 0u, W.bvh_width);
 
     const uint32_t n_waves = (uint32_t)waves.size();
     // Jobs completed by each wave: [done_lo[w], done_lo[w + 1]) (jobs are packed in order, so their last
@@ -1739,7 +1759,7 @@ extern "C" int pyre_render_noalloc(pyre_ctx* ctx, const pyre_scene* scene, const
     PathSoA S;
     carve_paths((char*)scratch, (size_t)W.npix * K, ns, W.npix, &S);
 
-    const Launch Lc = make_launch<false>(ctx, rp.block_size, W.bvh_width);
+    const Launch Lc = make_launch<false>(ctx, D, rp.block_size, W.bvh_width);
 
     cudaStream_t st = ctx->stream;
     // The array keeps the previous call's contents: clear the sums and counters.
@@ -2014,8 +2034,11 @@ extern "C" int pyre_backward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_
     W.smem_grad = mat_smem ? 1 : 0;
     const size_t smem = grad_smem_bytes(W.env_cache, mat_smem);
 
-    const Launch Lc = make_launch<false>(ctx, rp.block_size, W.bvh_width);
-    const int grid_adj = grid_for(ctx, k_shade<false, true>, Lc.block_stage, smem);
+    const Launch Lc = make_launch<false>(ctx, D, rp.block_size, W.bvh_width);
+    // one variant for every scene with quad lights: the adjoint kernels are the slowest to compile
+    const bool env_only = Lc.lights == SHADE_ENV;
+    const int grid_adj = env_only ? grid_for(ctx, k_shade<false, true, SHADE_ENV>, Lc.block_stage, smem)
+                                  : grid_for(ctx, k_shade<false, true, SHADE_QUADS | SHADE_ENV>, Lc.block_stage, smem);
     const int grid_acc = grid_for(ctx, k_accumulate_adjoint, Lc.block_stage, smem);
     PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.ctl, 0, sizeof(WaveCtl), st));
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0], st));
@@ -2025,7 +2048,8 @@ extern "C" int pyre_backward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_
         for (uint32_t d = 0; d < W.max_depth; ++d) {
             launch_extend<false>(st, Lc, D, S, W, d);
             if (W.sort) enqueue_sort(ctx, D, S, Lc, d, W.sort);
-            k_shade<false, true><<<grid_adj, Lc.block_stage, smem, st>>>(D, S, W, d);
+            if (env_only) k_shade<false, true, SHADE_ENV><<<grid_adj, Lc.block_stage, smem, st>>>(D, S, W, d);
+            else k_shade<false, true, SHADE_QUADS | SHADE_ENV><<<grid_adj, Lc.block_stage, smem, st>>>(D, S, W, d);
             if (W.ns > 0) launch_shadow<false>(st, Lc, D, S, W, d);
         }
         k_accumulate_adjoint<<<grid_acc, Lc.block_stage, smem, st>>>(D, S, W);
