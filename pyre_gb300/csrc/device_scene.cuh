@@ -346,9 +346,20 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
         --sp;
         return sp < SK ? sstack[sp][tid] : stack[sp - SK];
     };
-    bool drained = false;  // warp-uniform: the queue has no rays left
-    uint32_t next = 0, end = 0;  // warp-uniform: the rest of the warp's share of the queue
-    const uint32_t share = min((uint32_t)PYRE_SHARE, n / (gridDim.x * (blockDim.x >> 5) * 64u) & ~31u);
+    // A queue of less than 32 rays per warp is dealt out evenly: a warp runs the
+    // union of its rays' steps, so the launch's time is that of its fullest
+    // warp, and no warp waits for the counter. Small launches (the viewer's, a
+    // large wave's last bounces) are bound by that latency.
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    bool drained = false;         // warp-uniform: the counter has no rays left
+    uint32_t next = 0, end = 0;   // warp-uniform: the rest of the warp's share of the queue
+    if (n < 32u * warps) {
+        const uint32_t slice = (n + warps - 1) / warps;
+        next = min((blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * slice, n);
+        end = min(next + slice, n);
+        drained = true;
+    }
+    const uint32_t share = min((uint32_t)PYRE_SHARE, n / (warps * 64u) & ~31u);
     uint32_t id = 0;
     int node = PYRE_REF_NONE;
     int postponed = PYRE_REF_NONE;  // any hit: a leaf met while stepping on
