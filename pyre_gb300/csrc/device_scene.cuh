@@ -320,9 +320,35 @@ __device__ __forceinline__ bool slab2(pair32 loxy, pair32 hixy, pair32 z, pair32
 #ifndef PYRE_STACK_SHARED
 #define PYRE_STACK_SHARED 12
 #endif
+// Shared memory of a block of at most 128 threads (a closest-hit kernel's, or
+// an any-hit kernel's, which keeps no hit).
+template <bool ANY>
+struct TraceShared {
+    int stack[PYRE_STACK_SHARED][128];  // bottom entries of the stacks
+    float ray[8][128];                  // o, d, time, job
+    int hit[ANY ? 1 : 4][128];          // u, v, instance slot, triangle slot
+};
+// Who traces a queue: warp `warp` of `warps` (all others of the grid stay
+// out). With `deal`, the queue holds less than 32 rays for each of them and is
+// dealt out evenly: a warp runs the union of its rays' steps, so the launch's
+// time is that of its fullest warp, and no warp waits for the counter. Short
+// queues (the viewer's, a large wave's last bounces) are bound by that latency.
+struct TraceTeam {
+    uint32_t warp, warps;
+    bool deal;
+};
+__device__ __forceinline__ TraceTeam whole_grid(uint32_t n) {
+    TraceTeam t;
+    t.warps = gridDim.x * (blockDim.x >> 5);
+    t.warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    t.deal = n < 32u * t.warps;
+    return t;
+}
+
 template <bool ANY, class Src>
 __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
-                                             int refill) {
+                                             int refill, const TraceTeam& team, int (*sstack)[128], float (*sray)[128],
+                                             int (*shit)[128]) {
     constexpr int LEAF_WAIT = ANY ? PYRE_LEAF_WAIT_ANY : PYRE_LEAF_WAIT_CLOSEST;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -331,9 +357,6 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
     // leaf's sibling waiting for the leaf
     constexpr int STACK = PYRE_STACK + 4;
     constexpr int SK = PYRE_STACK_SHARED;
-    __shared__ int sstack[SK][128];  // blocks have at most 128 threads
-    __shared__ float sray[8][128];          // o, d, time, job
-    __shared__ int shit[ANY ? 1 : 4][128];  // u, v, instance slot, triangle slot
     const int tid = threadIdx.x;
     int stack[STACK - SK + 1];  // + 1: the node that waits while a postponed leaf is tested
     int sp = 0;
@@ -346,20 +369,15 @@ __device__ __forceinline__ void trace_binary(const DevScene& S, const Src& src, 
         --sp;
         return sp < SK ? sstack[sp][tid] : stack[sp - SK];
     };
-    // A queue of less than 32 rays per warp is dealt out evenly: a warp runs the
-    // union of its rays' steps, so the launch's time is that of its fullest
-    // warp, and no warp waits for the counter. Small launches (the viewer's, a
-    // large wave's last bounces) are bound by that latency.
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     bool drained = false;         // warp-uniform: the counter has no rays left
     uint32_t next = 0, end = 0;   // warp-uniform: the rest of the warp's share of the queue
-    if (n < 32u * warps) {
-        const uint32_t slice = (n + warps - 1) / warps;
-        next = min((blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * slice, n);
+    if (team.deal) {
+        const uint32_t slice = (n + team.warps - 1) / team.warps;
+        next = min(team.warp * slice, n);
         end = min(next + slice, n);
         drained = true;
     }
-    const uint32_t share = min((uint32_t)PYRE_SHARE, n / (warps * 64u) & ~31u);
+    const uint32_t share = min((uint32_t)PYRE_SHARE, n / (team.warps * 64u) & ~31u);
     uint32_t id = 0;
     int node = PYRE_REF_NONE;
     int postponed = PYRE_REF_NONE;  // any hit: a leaf met while stepping on
@@ -894,8 +912,10 @@ __device__ __forceinline__ bool quad_intersect(const DevQuadLight& L, const f3& 
 template <bool ANY, int WIDTH, class Src>
 __device__ __forceinline__ void trace_stream(const DevScene& S, const Src& src, uint32_t n, uint32_t* counter,
                                              int refill) {
-    if constexpr (WIDTH == 2) trace_binary<ANY>(S, src, n, counter, refill);
-    else trace_wide<ANY, WIDTH>(S, src, n, counter, refill);
+    if constexpr (WIDTH == 2) {
+        __shared__ TraceShared<ANY> sh;
+        trace_binary<ANY>(S, src, n, counter, refill, whole_grid(n), sh.stack, sh.ray, sh.hit);
+    } else trace_wide<ANY, WIDTH>(S, src, n, counter, refill);
 }
 
 // Quad lights after primitives with strict `<` (scene.rs:78-94): lights
