@@ -167,20 +167,33 @@ __device__ __forceinline__ T warp_sum(T v) {
 #ifndef PYRE_ENV_CACHE_DIRECT
 #define PYRE_ENV_CACHE_DIRECT 1
 #endif
-// Material terms: lanes that hold the same material (most of a warp once the
-// backward sorts its paths by material) are summed with full-warp FP32
-// butterflies, and one lane adds each sum to the block's FP64 sums in shared
-// memory; other lanes add their own terms. The backward of the 512^2 problem
-// took 19.3 ms, against 19.7 with FP64 butterflies and 20.0 with every lane
-// adding to the FP64 sums (PYRE_MAT_DIRECT; before the material sort that
-// was the fastest: 23.9 against 24.6 ms). A warp sums at most 32 terms in
-// FP32; the sums over the block and the image stay FP64.
-#ifndef PYRE_MAT_WARP32
-#define PYRE_MAT_WARP32 1
-#endif
-#ifndef PYRE_MAT_DIRECT
-#define PYRE_MAT_DIRECT 0
-#endif
+// The six parameter terms of the lanes with `mine`, summed over the warp in
+// FP64 (all 32 lanes call it): each of the first three steps halves the values
+// a lane carries, so a sum takes 9 additions and exchanges instead of 30, and
+// the sums end on six lanes, which add them to the block's sums side by side.
+// *k gets the lane's parameter, PYRE_NPARAM or more where it holds none. FP32
+// butterflies per parameter (each warp's sum rounded to 24 bits) took 14.14
+// against 13.99 ms of backward on the 512^2 problem, FP64 ones 14.7; the
+// material gradients now repeat to 1e-15 between runs instead of 1e-7.
+__device__ __forceinline__ double warp_sum6(bool mine, const float (&g)[PYRE_NPARAM], int* k) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    const float z = 0.0f;
+    const float f[8] = {mine ? g[0] : z, mine ? g[1] : z, mine ? g[2] : z, mine ? g[3] : z,
+                        mine ? g[4] : z, mine ? g[5] : z, z, z};
+    double w4[4], w2[2];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        w4[q] = (double)(b4 ? f[4 + q] : f[q]) + (double)__shfl_xor_sync(FULL, b4 ? f[q] : f[4 + q], 16);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) w2[q] = (b3 ? w4[2 + q] : w4[q]) + __shfl_xor_sync(FULL, b3 ? w4[q] : w4[2 + q], 8);
+    double v = (b2 ? w2[1] : w2[0]) + __shfl_xor_sync(FULL, b2 ? w2[0] : w2[1], 4);
+    v += __shfl_xor_sync(FULL, v, 2);
+    v += __shfl_xor_sync(FULL, v, 1);
+    *k = (lane & 3) == 0 ? (b4 ? 4 : 0) + (b3 ? 2 : 0) + (b2 ? 1 : 0) : PYRE_NPARAM;
+    return v;
+}
 
 // A block's gradient accumulators in its dynamic shared memory: the texel
 // cache (null without texel gradients), then the material sums (null when
@@ -324,13 +337,6 @@ __device__ __forceinline__ void warp_flush(const DevScene& S, float* env_grad, d
     };
     // materials
     bool left = t.mat != PYRE_NO_KEY;
-#if PYRE_MAT_DIRECT
-    if (G.mat) {  // the block's FP64 sums in shared memory take each lane's terms directly
-        if (left)
-            for (int k = 0; k < PYRE_NPARAM; ++k) mat_add(t.mat, k, (double)t.g[k]);
-        left = false;
-    }
-#endif
     if (full && __any_sync(FULL, left)) {
         // only keys that several lanes hold are worth a butterfly
         const unsigned peers = __match_any_sync(FULL, t.mat);
@@ -340,15 +346,9 @@ __device__ __forceinline__ void warp_flush(const DevScene& S, float* env_grad, d
             const uint32_t key = __shfl_sync(FULL, t.mat, src);
             const bool mine = left && t.mat == key;
             todo &= ~__ballot_sync(FULL, mine);
-#pragma unroll
-            for (int k = 0; k < PYRE_NPARAM; ++k) {
-#if PYRE_MAT_WARP32
-                const double v = (double)warp_sum(mine ? t.g[k] : 0.0f);
-#else
-                const double v = warp_sum(mine ? (double)t.g[k] : 0.0);
-#endif
-                if (lane == src) mat_add(key, k, v);
-            }
+            int k;
+            const double v = warp_sum6(mine, t.g, &k);
+            if (k < PYRE_NPARAM) mat_add(key, k, v);
             if (mine) left = false;
         }
     }
