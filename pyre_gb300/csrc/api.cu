@@ -63,11 +63,7 @@ int ensure_workspace(pyre_ctx* ctx, Workspace& ws, size_t bytes) {
     return PYRE_OK;
 }
 
-int take_kernel_error(pyre_ctx* ctx) {
-    int flag = 0;
-    cudaError_t e = cudaMemcpyAsync(&flag, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return cuda_check(ctx, e, "reading the kernel status");
+int kernel_error(pyre_ctx* ctx, int flag) {
     if (flag != 0) {
         cudaMemsetAsync(ctx->d_error, 0, sizeof(int), ctx->stream);
         cudaStreamSynchronize(ctx->stream);
@@ -379,6 +375,8 @@ int pyre_ctx_create(int device, pyre_ctx** out) {
     if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaMalloc(&ctx->d_error, sizeof(int))) != cudaSuccess ||
         (e = cudaMalloc(&ctx->d_counter, 64 * sizeof(unsigned int))) != cudaSuccess ||
+        (e = cudaMalloc(&ctx->d_status, sizeof(DeviceStatus))) != cudaSuccess ||
+        (e = cudaMallocHost(&ctx->h_stage, PYRE_STAGE_BYTES + sizeof(DeviceStatus))) != cudaSuccess ||
         (e = cudaMemset(ctx->d_error, 0, sizeof(int))) != cudaSuccess) {
         int rc = cuda_check(nullptr, e, "pyre_ctx_create");
         pyre_ctx_destroy(ctx);
@@ -400,6 +398,8 @@ int pyre_ctx_destroy(pyre_ctx* ctx) {
     if (ctx->prog_ws.ptr) cudaFree(ctx->prog_ws.ptr);
     if (ctx->d_error) cudaFree(ctx->d_error);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
+    if (ctx->d_status) cudaFree(ctx->d_status);
+    if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
     for (auto& ev : ctx->ev)
         if (ev) cudaEventDestroy(ev);
     for (cudaEvent_t ev : ctx->stage_ev) cudaEventDestroy(ev);

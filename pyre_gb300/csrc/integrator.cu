@@ -235,7 +235,7 @@ __device__ __forceinline__ uint32_t find_segment(const DevSeg* segs, const DevWa
     return lo;
 }
 
-__global__ void k_wave_end(WaveCtl* ctl, uint32_t max_depth) {
+__global__ void k_wave_end(WaveCtl* ctl, uint32_t max_depth, const int* error_flag, DeviceStatus* status) {
     if (threadIdx.x != 0) return;
     unsigned long long e = 0, s = 0;
     for (uint32_t d = 0; d < max_depth; ++d) { e += ctl->count[d]; s += ctl->scount[d]; }
@@ -243,6 +243,10 @@ __global__ void k_wave_end(WaveCtl* ctl, uint32_t max_depth) {
     ctl->shadow_rays += s;
     ctl->samples += ctl->n_valid;
     ctl->wave += 1;
+    status->samples = ctl->samples;  // totals of the call so far
+    status->extend_rays = ctl->extend_rays;
+    status->shadow_rays = ctl->shadow_rays;
+    status->error = *error_flag;
 }
 
 // Path order of a wave (or batch segment) that holds K samples of every pixel
@@ -1075,8 +1079,8 @@ namespace {
 
 template <typename K>
 int grid_for(pyre_ctx* ctx, K kernel, int block, size_t smem = 0) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+    int& per_sm = ctx->blocks_per_sm[{(const void*)kernel, (size_t)block << 32 | smem}];
+    if (!per_sm) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
     return std::max(1, per_sm) * std::max(1, ctx->num_sms);
 }
 
@@ -1130,8 +1134,10 @@ size_t carve_paths(char* base, size_t P, uint32_t ns, uint32_t npix, PathSoA* ou
 // 8 Mi and 128 Mi paths. On the 1080p 64-spp studio frame 8, 16, 32, 64 and
 // 128 Mi paths gave 444, 479, 497, 506 and 510 Msamples/s: the last bounces
 // of a wave hold few live paths, and a larger wave spends a smaller share of
-// those launches draining the warps' final rays.
-uint64_t default_wave_paths(pyre_ctx* ctx, uint32_t ns, bool batch, bool adjoint) {
+// those launches draining the warps' final rays. A call of at most 8 Mi paths
+// (all) fits any of these and does not ask for the free memory.
+uint64_t default_wave_paths(pyre_ctx* ctx, uint32_t ns, bool batch, bool adjoint, uint64_t all) {
+    if (all <= (uint64_t)8 << 20) return (uint64_t)8 << 20;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
@@ -1261,7 +1267,8 @@ void enqueue_sort(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const Laun
     k_sort_scatter<<<Lc.grid_sort, 256, 0, st>>>(S, P, d);
 }
 
-void enqueue_wave(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const WaveParams& W, const Launch& Lc) {
+void enqueue_wave(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const WaveParams& W, const Launch& Lc,
+                  DeviceStatus* status) {
     cudaStream_t st = ctx->stream;
     mark(ctx, STAGE_OTHER);
     k_wave_begin<<<1, 32, 0, st>>>(P.ctl, W.spp_begin, W.spp_end, W.k_per_wave, W.npix);
@@ -1276,7 +1283,7 @@ void enqueue_wave(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const Wave
     }
     mark(ctx, STAGE_OTHER);
     k_accumulate<<<Lc.grid_acc, Lc.block_stage, 0, st>>>(P, W);
-    k_wave_end<<<1, 32, 0, st>>>(P.ctl, W.max_depth);
+    k_wave_end<<<1, 32, 0, st>>>(P.ctl, W.max_depth, S.error_flag, status);
     mark(ctx, STAGE_END);
 }
 
@@ -1297,7 +1304,7 @@ void enqueue_wave_batch(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, cons
     }
     mark(ctx, STAGE_OTHER);
     k_accumulate_batch<<<Lc.grid_acc, Lc.block_stage, 0, st>>>(P, W);
-    k_wave_end<<<1, 32, 0, st>>>(P.ctl, W.max_depth);
+    k_wave_end<<<1, 32, 0, st>>>(P.ctl, W.max_depth, S.error_flag, ctx->d_status);
     mark(ctx, STAGE_END);
 }
 
@@ -1307,6 +1314,33 @@ uint32_t kernels_per_wave(const pyre_ctx* ctx, const WaveParams& W) {
     // extend at depth 0, then per depth the sorts, shade, the shadow rays and the next depth's extend rays
     const uint32_t traces = W.ns == 0 ? W.max_depth : one_trace_launch(ctx, W) ? W.max_depth + 1 : 2 * W.max_depth;
     return 4 + W.max_depth * (sorts + 1) + traces;
+}
+
+// Clears the film sums and the wave counters: consecutive arrays (carve_paths), one memset.
+int clear_sums(pyre_ctx* ctx, const PathSoA& S) {
+    const size_t bytes = (size_t)((const char*)(S.ctl + 1) - (const char*)S.acc_r);
+    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_r, 0, bytes, ctx->stream));
+    return PYRE_OK;
+}
+
+// Ends a call: `bytes` of results from `src` on the device, and the status
+// behind them, into the context's pinned buffer with one copy.
+int read_back(pyre_ctx* ctx, const char* src, size_t bytes, DeviceStatus* status) {
+    PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_stage, src, bytes + sizeof(DeviceStatus), cudaMemcpyDeviceToHost, ctx->stream));
+    PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    std::memcpy(status, ctx->h_stage + bytes, sizeof(DeviceStatus));
+    return PYRE_OK;
+}
+
+void fill_stats(pyre_ctx* ctx, const DeviceStatus& d, uint32_t waves, uint32_t launches) {
+    pyre_render_stats& s = ctx->stats;
+    std::memset(&s, 0, sizeof s);
+    s.samples = d.samples;
+    s.extend_rays = d.extend_rays;
+    s.shadow_rays = d.shadow_rays;
+    s.waves = waves;
+    s.kernel_launches = launches;
+    cudaEventElapsedTime(&s.ms_total, ctx->ev[0], ctx->ev[1]);
 }
 
 // Largest pixel count of one view: path and pixel indices are 32-bit, and a
@@ -1413,7 +1447,7 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
     rc = select_bvh(ctx, const_cast<pyre_scene*>(scene), rp.bvh_width, &D, &W.bvh_width);
     if (rc) return rc;
     const uint32_t spp = rp.spp_end - rp.spp_begin;
-    uint64_t target = rp.wave_paths ? rp.wave_paths : default_wave_paths(ctx, W.ns, false, false);
+    uint64_t target = rp.wave_paths ? rp.wave_paths : default_wave_paths(ctx, W.ns, false, false, (uint64_t)npix * spp);
     uint64_t K = std::max<uint64_t>(1, target / W.npix);
     K = std::min<uint64_t>(K, spp);
     if ((uint64_t)W.npix * K > (uint64_t)1 << 31) K = std::max<uint64_t>(1, ((uint64_t)1 << 31) / W.npix);
@@ -1428,19 +1462,22 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
     PathSoA S;
     carve_paths((char*)ctx->render_ws.ptr, P, std::max(W.ns, 1u), W.npix, &S);
     S.keep_L = keep;
-    if (film->mem == PYRE_MEM_HOST && (rc = ensure_workspace(ctx, ctx->io_ws, film_bytes))) return rc;
+    if (film->mem == PYRE_MEM_HOST && (rc = ensure_workspace(ctx, ctx->io_ws, film_bytes + sizeof(DeviceStatus))))
+        return rc;
 
     const Launch Lc = make_launch<false>(ctx, D, rp.block_size, W.bvh_width);
 
     cudaStream_t st = ctx->stream;
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_r, 0, (size_t)W.npix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_a, 0, (size_t)W.npix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_n, 0, (size_t)W.npix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.ctl, 0, sizeof(WaveCtl), st));
+    if ((rc = clear_sums(ctx, S))) return rc;
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0], st));
 
     ctx->stage_used = 0;
-    if (rp.use_graph && !ctx->stage_timing && !keep && !prog) {
+    const bool graph = rp.use_graph && !ctx->stage_timing && !keep && !prog;
+    // a small host film and the status come back together, through the pinned buffer
+    const bool staged = film->mem == PYRE_MEM_HOST && !graph && film_bytes <= PYRE_STAGE_BYTES;
+    float* staging = (float*)ctx->io_ws.ptr;
+    DeviceStatus* d_status = staged ? (DeviceStatus*)((char*)staging + film_bytes) : ctx->d_status;
+    if (graph) {
         // One wave captured once per configuration, replayed `waves` times.
         char key[256];
         std::snprintf(key, sizeof key, "%llu/%p/%u/%u/%u/%u/%u/%u/%u/%u/%d/r%d/s%d/w%d",
@@ -1456,7 +1493,7 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
             if (ctx->wave_graph) { cudaGraphExecDestroy(ctx->wave_graph); ctx->wave_graph = nullptr; }
             cudaGraph_t g;
             PYRE_CUDA_TRY(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            enqueue_wave(ctx, D, S, W, Lc);
+            enqueue_wave(ctx, D, S, W, Lc, ctx->d_status);
             PYRE_CUDA_TRY(ctx, cudaStreamEndCapture(st, &g));
             cudaError_t e = cudaGraphInstantiate(&ctx->wave_graph, g, 0);
             cudaGraphDestroy(g);
@@ -1465,37 +1502,31 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
         }
         for (uint32_t w = 0; w < waves; ++w) PYRE_CUDA_TRY(ctx, cudaGraphLaunch(ctx->wave_graph, st));
     } else {
-        for (uint32_t w = 0; w < waves; ++w) enqueue_wave(ctx, D, S, W, Lc);
+        for (uint32_t w = 0; w < waves; ++w) enqueue_wave(ctx, D, S, W, Lc, d_status);
     }
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
 
     const float inv_spp = 1.0f / (float)spp;
     float* out[4] = {prog ? nullptr : film->radiance, film->albedo, film->normal, film->depth};
     float* dst[4];
-    float* staging = (float*)ctx->io_ws.ptr;
     size_t offs[4] = {0, (size_t)W.npix * 3, (size_t)W.npix * 6, (size_t)W.npix * 9};
     for (int c = 0; c < 4; ++c) dst[c] = out[c] ? (film->mem == PYRE_MEM_HOST ? staging + offs[c] : out[c]) : nullptr;
     k_finalize<<<Lc.grid_acc, 256, 0, st>>>(S, W.npix, inv_spp, dst[0], dst[1], dst[2], dst[3]);
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], st));
-    if (film->mem == PYRE_MEM_HOST) {
+    auto channel_bytes = [&](int c) { return (c == 3 ? 1 : 3) * (size_t)W.npix * sizeof(float); };
+    if (film->mem == PYRE_MEM_HOST && !staged) {
         for (int c = 0; c < 4; ++c)
-            if (out[c])
-                PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(out[c], dst[c], (c == 3 ? 1 : 3) * (size_t)W.npix * sizeof(float),
-                                                   cudaMemcpyDeviceToHost, st));
+            if (out[c]) PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(out[c], dst[c], channel_bytes(c), cudaMemcpyDeviceToHost, st));
     }
-    WaveCtl ctl;
-    PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(&ctl, S.ctl, sizeof ctl, cudaMemcpyDeviceToHost, st));
-    PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if ((rc = take_kernel_error(ctx))) return rc;
+    DeviceStatus ds;
+    if ((rc = read_back(ctx, staged ? (const char*)staging : (const char*)d_status, staged ? film_bytes : 0, &ds))) return rc;
+    if ((rc = kernel_error(ctx, ds.error))) return rc;
+    if (staged)
+        for (int c = 0; c < 4; ++c)
+            if (out[c]) std::memcpy(out[c], ctx->h_stage + offs[c] * sizeof(float), channel_bytes(c));
+    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W) + 1);
     pyre_render_stats& s = ctx->stats;
-    std::memset(&s, 0, sizeof s);
-    s.samples = ctl.samples;
-    s.extend_rays = ctl.extend_rays;
-    s.shadow_rays = ctl.shadow_rays;
-    s.waves = waves;
-    s.kernel_launches = waves * kernels_per_wave(ctx, W) + 1;
-    cudaEventElapsedTime(&s.ms_total, ctx->ev[0], ctx->ev[1]);
     if (ctx->stage_timing) {
         float acc[4] = {0, 0, 0, 0};
         for (size_t k = 0; k + 1 < ctx->stage_used; ++k) {
@@ -1561,7 +1592,7 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
     if (total_pix > 0x7fffffffull) return set_error(ctx, PYRE_ERR_INVALID, "pyre_render_batch: too many pixels");
 
     // ---- wave plan: jobs packed in order, each job's samples in order
-    uint64_t cap = wave_paths ? wave_paths : default_wave_paths(ctx, scene->part_light_max, true, false);
+    uint64_t cap = wave_paths ? wave_paths : default_wave_paths(ctx, scene->part_light_max, true, false, total_samples);
     cap = std::min<uint64_t>(std::max<uint64_t>(cap, max_npix), (uint64_t)1 << 31);
     std::vector<DevSeg> segs;
     std::vector<DevWave> waves;
@@ -1626,10 +1657,7 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
     PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_jobs, dj.data(), job_bytes, cudaMemcpyHostToDevice, st));
     PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_segs, segs.data(), seg_bytes, cudaMemcpyHostToDevice, st));
     PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_waves, waves.data(), wave_bytes, cudaMemcpyHostToDevice, st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_r, 0, total_pix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_a, 0, total_pix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_n, 0, total_pix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.ctl, 0, sizeof(WaveCtl), st));
+    if ((rc = clear_sums(ctx, S))) return rc;
 
     const Launch Lc = make_launch<true>(ctx, D, params ? params->block_size : 0u, W.bvh_width);
 
@@ -1707,18 +1735,10 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
         }
     }
     PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(cst));
-    WaveCtl ctl;
-    PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(&ctl, S.ctl, sizeof ctl, cudaMemcpyDeviceToHost, st));
-    PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if ((rc = take_kernel_error(ctx))) return rc;
-    pyre_render_stats& s = ctx->stats;
-    std::memset(&s, 0, sizeof s);
-    s.samples = ctl.samples;
-    s.extend_rays = ctl.extend_rays;
-    s.shadow_rays = ctl.shadow_rays;
-    s.waves = n_waves;
-    s.kernel_launches = n_waves * kernels_per_wave(ctx, W) + finalizes;
-    cudaEventElapsedTime(&s.ms_total, ctx->ev[0], ctx->ev[1]);
+    DeviceStatus ds;
+    if ((rc = read_back(ctx, (const char*)ctx->d_status, 0, &ds))) return rc;
+    if ((rc = kernel_error(ctx, ds.error))) return rc;
+    fill_stats(ctx, ds, n_waves, n_waves * kernels_per_wave(ctx, W) + finalizes);
     return PYRE_OK;
 }
 
@@ -1820,32 +1840,21 @@ extern "C" int pyre_render_noalloc(pyre_ctx* ctx, const pyre_scene* scene, const
 
     cudaStream_t st = ctx->stream;
     // The array keeps the previous call's contents: clear the sums and counters.
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_r, 0, (size_t)W.npix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_a, 0, (size_t)W.npix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.acc_n, 0, (size_t)W.npix * sizeof(float4), st));
-    PYRE_CUDA_TRY(ctx, cudaMemsetAsync(S.ctl, 0, sizeof(WaveCtl), st));
+    if ((rc = clear_sums(ctx, S))) return rc;
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0], st));
     const int timing = ctx->stage_timing;
     ctx->stage_timing = 0;  // stage timing would create events
-    for (uint32_t w = 0; w < waves; ++w) enqueue_wave(ctx, D, S, W, Lc);
+    for (uint32_t w = 0; w < waves; ++w) enqueue_wave(ctx, D, S, W, Lc, ctx->d_status);
     ctx->stage_timing = timing;
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
     k_finalize<<<Lc.grid_acc, 256, 0, st>>>(S, W.npix, 1.0f / (float)spp, film->radiance, film->albedo, film->normal,
                                               film->depth);
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], st));
-    WaveCtl ctl;
-    PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(&ctl, S.ctl, sizeof ctl, cudaMemcpyDeviceToHost, st));
-    PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if ((rc = take_kernel_error(ctx))) return rc;
-    pyre_render_stats& s = ctx->stats;
-    std::memset(&s, 0, sizeof s);
-    s.samples = ctl.samples;
-    s.extend_rays = ctl.extend_rays;
-    s.shadow_rays = ctl.shadow_rays;
-    s.waves = waves;
-    s.kernel_launches = waves * kernels_per_wave(ctx, W) + 1;
-    cudaEventElapsedTime(&s.ms_total, ctx->ev[0], ctx->ev[1]);
+    DeviceStatus ds;
+    if ((rc = read_back(ctx, (const char*)ctx->d_status, 0, &ds))) return rc;
+    if ((rc = kernel_error(ctx, ds.error))) return rc;
+    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W) + 1);
     return PYRE_OK;
 }
 
@@ -1885,10 +1894,12 @@ static int intersect_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_ray
     int32_t *kind = nullptr, *inst = nullptr, *tri = nullptr;
     float *tt = nullptr, *uu = nullptr, *vv = nullptr;
     uint8_t* occ = occluded;
+    const size_t in_bytes = n * (time ? 9 : 8) * sizeof(float), out_bytes = any ? n : n * 6 * sizeof(float);
+    // small host queries: one copy of packed rays in, one of packed results (and the kernel status) out
+    const size_t out_at = (in_bytes + 7) & ~(size_t)7, status_at = (out_bytes + 7) & ~(size_t)7;
+    const bool staged = mem == PYRE_MEM_HOST && out_at + status_at <= PYRE_STAGE_BYTES;
     if (!any) { kind = hits->kind; inst = hits->instance; tri = hits->triangle; tt = hits->t; uu = hits->u; vv = hits->v; }
     if (mem == PYRE_MEM_HOST) {
-        size_t in_bytes = n * (time ? 9 : 8) * sizeof(float);
-        size_t out_bytes = any ? n : n * 6 * sizeof(float);
         int rc = ensure_workspace(ctx, ctx->io_ws, in_bytes + out_bytes + 1024);
         if (rc) return rc;
         char* b = (char*)ctx->io_ws.ptr;
@@ -1897,12 +1908,18 @@ static int intersect_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_ray
         float* d_tmin = d_dir + 3 * n;
         float* d_tmax = d_tmin + n;
         float* d_time = time ? d_tmax + n : nullptr;
-        char* ob = (char*)(d_tmax + n + (time ? n : 0));
-        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_org, org, 3 * n * sizeof(float), cudaMemcpyHostToDevice, st));
-        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_dir, dir, 3 * n * sizeof(float), cudaMemcpyHostToDevice, st));
-        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_tmin, tmin, n * sizeof(float), cudaMemcpyHostToDevice, st));
-        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_tmax, tmax, n * sizeof(float), cudaMemcpyHostToDevice, st));
-        if (time) PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(d_time, time, n * sizeof(float), cudaMemcpyHostToDevice, st));
+        char* ob = b + out_at;
+        const struct { float* dst; const float* src; size_t count; } in[5] = {
+            {d_org, org, 3 * n}, {d_dir, dir, 3 * n}, {d_tmin, tmin, n}, {d_tmax, tmax, n}, {d_time, time, time ? n : 0}};
+        if (staged) {
+            for (const auto& a : in)
+                if (a.count) std::memcpy(ctx->h_stage + ((char*)a.dst - b), a.src, a.count * sizeof(float));
+            PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(b, ctx->h_stage, in_bytes, cudaMemcpyHostToDevice, st));
+        } else {
+            for (const auto& a : in)
+                if (a.count)
+                    PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(a.dst, a.src, a.count * sizeof(float), cudaMemcpyHostToDevice, st));
+        }
         org = d_org; dir = d_dir; tmin = d_tmin; tmax = d_tmax; time = d_time;
         if (any) occ = (uint8_t*)ob;
         else {
@@ -1920,7 +1937,21 @@ static int intersect_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_ray
     else launch_intersect<false>(ctx, D, q, (uint32_t)n, width);
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], st));
-    if (mem == PYRE_MEM_HOST) {
+    if (staged) {
+        char* h = ctx->h_stage;
+        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(h, any ? (const char*)occ : (const char*)kind, out_bytes, cudaMemcpyDeviceToHost, st));
+        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(h + status_at, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        int flag;
+        std::memcpy(&flag, h + status_at, sizeof flag);
+        if (int rc = kernel_error(ctx, flag)) return rc;
+        if (any) std::memcpy(occluded, h, n);
+        else {
+            const size_t q = n * 4;
+            std::memcpy(hits->kind, h, q); std::memcpy(hits->instance, h + q, q); std::memcpy(hits->triangle, h + 2 * q, q);
+            std::memcpy(hits->t, h + 3 * q, q); std::memcpy(hits->u, h + 4 * q, q); std::memcpy(hits->v, h + 5 * q, q);
+        }
+    } else if (mem == PYRE_MEM_HOST) {
         if (any) PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(occluded, occ, n, cudaMemcpyDeviceToHost, st));
         else {
             PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(hits->kind, kind, n * 4, cudaMemcpyDeviceToHost, st));
@@ -1931,8 +1962,12 @@ static int intersect_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_ray
             PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(hits->v, vv, n * 4, cudaMemcpyDeviceToHost, st));
         }
     }
-    PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if (int rc = take_kernel_error(ctx)) return rc;
+    if (!staged) {
+        int* flag = (int*)ctx->h_stage;
+        PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(flag, ctx->d_error, sizeof(int), cudaMemcpyDeviceToHost, st));
+        PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+        if (int rc = kernel_error(ctx, *flag)) return rc;
+    }
     // statistics: the query kernel's device time and its ray count
     pyre_render_stats& s = ctx->stats;
     std::memset(&s, 0, sizeof s);
@@ -2051,7 +2086,7 @@ extern "C" int pyre_backward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_
     if ((rc = select_bvh(ctx, const_cast<pyre_scene*>(scene), rp.bvh_width, &D, &W.bvh_width))) return rc;
     const uint32_t spp = rp.spp_end - rp.spp_begin;
     uint64_t K = std::max<uint64_t>(
-        1, (rp.wave_paths ? rp.wave_paths : default_wave_paths(ctx, W.ns, false, true)) / W.npix);
+        1, (rp.wave_paths ? rp.wave_paths : default_wave_paths(ctx, W.ns, false, true, (uint64_t)npix * spp)) / W.npix);
     K = std::min<uint64_t>(K, spp);
     if ((uint64_t)W.npix * K > (uint64_t)1 << 31) K = std::max<uint64_t>(1, ((uint64_t)1 << 31) / W.npix);
     W.k_per_wave = (uint32_t)K;
@@ -2110,7 +2145,7 @@ extern "C" int pyre_backward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_
             launch_traces<false>(ctx, Lc, D, S, W, d);
         }
         k_accumulate_adjoint<<<grid_acc, Lc.block_stage, smem, st>>>(D, S, W);
-        k_wave_end<<<1, 32, 0, st>>>(S.ctl, W.max_depth);
+        k_wave_end<<<1, 32, 0, st>>>(S.ctl, W.max_depth, D.error_flag, ctx->d_status);
     }
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
     PYRE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], st));
@@ -2120,17 +2155,9 @@ extern "C" int pyre_backward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_
         if (grads->env && env_elems)
             PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(grads->env, d_env, env_elems * 4, cudaMemcpyDeviceToHost, st));
     }
-    WaveCtl ctl;
-    PYRE_CUDA_TRY(ctx, cudaMemcpyAsync(&ctl, S.ctl, sizeof ctl, cudaMemcpyDeviceToHost, st));
-    PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if ((rc = take_kernel_error(ctx))) return rc;
-    pyre_render_stats& s = ctx->stats;
-    std::memset(&s, 0, sizeof s);
-    s.samples = ctl.samples;
-    s.extend_rays = ctl.extend_rays;
-    s.shadow_rays = ctl.shadow_rays;
-    s.waves = waves;
-    s.kernel_launches = waves * kernels_per_wave(ctx, W);
-    cudaEventElapsedTime(&s.ms_total, ctx->ev[0], ctx->ev[1]);
+    DeviceStatus ds;
+    if ((rc = read_back(ctx, (const char*)ctx->d_status, 0, &ds))) return rc;
+    if ((rc = kernel_error(ctx, ds.error))) return rc;
+    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W));
     return PYRE_OK;
 }
