@@ -57,7 +57,7 @@ struct DeviceStatus {
 // about 8 us however small it is, and a small call makes a handful of them:
 // 4096 host rays 74 against 136 us, a 64x64 render with 4 samples 304 against
 // 380 us (with the occupancy and free-memory queries of each call gone).
-#define PYRE_STAGE_BYTES ((size_t)1 << 20)
+#define PYRE_STAGE_BYTES ((size_t)1 << 18)
 
 struct pyre_ctx {
     int device = 0;
