@@ -396,6 +396,7 @@ int pyre_ctx_destroy(pyre_ctx* ctx) {
     if (ctx->io_ws.ptr) cudaFree(ctx->io_ws.ptr);
     if (ctx->tape_ws.ptr) cudaFree(ctx->tape_ws.ptr);
     if (ctx->prog_ws.ptr) cudaFree(ctx->prog_ws.ptr);
+    if (ctx->build_ws.ptr) cudaFree(ctx->build_ws.ptr);
     if (ctx->d_error) cudaFree(ctx->d_error);
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->d_status) cudaFree(ctx->d_status);

@@ -72,6 +72,7 @@ struct pyre_ctx {
     Workspace render_ws;        // path state of the wavefront integrator
     Workspace io_ws;            // staging for host-memory rays / films
     Workspace tape_ws;          // pyre_forward: per-path radiance for pyre_backward
+    Workspace build_ws;         // arrays of the GPU BVH build
     Workspace prog_ws;          // pyre_render_progressive: device copy of a host running mean
     int bvh_builder = PYRE_BVH_BUILDER_HOST;  // where pyre_scene_upload builds instance BVHs
     int64_t fail_alloc_countdown = -1;  // pyre_inject_alloc_failure: allocations until one fails
