@@ -298,51 +298,55 @@ __device__ __forceinline__ TilePixel tile_pixel(uint32_t cw, uint32_t ch, uint32
     return t;
 }
 
-// main.rs:261-273: seed, jitter, ndc, lens, time, Camera::generate_ray.
+// main.rs:261-273: seed, jitter, ndc, lens, time, Camera::generate_ray, for path
+// i of a wave whose samples start at s_base, kv of them.
+template <bool BATCH>
+__device__ __forceinline__ void raygen_path(const PathSoA& P, const WaveParams& W, uint32_t s_base, uint32_t kv, uint32_t i) {
+    uint32_t x, y, s, width, height, max_depth = W.max_depth, job = 0;
+    const DevCamera* cam = &W.cam;
+    if (BATCH) {
+        const DevWave& wv = W.waves[P.ctl->wave];
+        const DevSeg sg = W.segs[find_segment(W.segs, wv, i, false)];
+        const DevJob& J = W.jobs[sg.job];
+        const TilePixel t = tile_pixel(J.width, J.height, sg.s_count, i - sg.path_base);
+        x = t.x; y = t.y; s = sg.s_first + t.k;
+        width = J.width; height = J.height;
+        max_depth = J.max_depth;
+        cam = &J.cam;
+        job = sg.job;
+    } else {
+        const TilePixel t = tile_pixel(W.cw, W.ch, kv, i);
+        x = W.cx0 + t.x; y = W.cy0 + t.y; s = s_base + t.k;
+        width = W.width; height = W.height;
+    }
+    Rng g;
+    g.seed(pixel_seed(x, y, s));
+    float jx = g.next_f32(), jy = g.next_f32();
+    f2 ndc;
+    ndc.x = 2.0f * ((float)x + jx) / (float)width - 1.0f;
+    ndc.y = 1.0f - 2.0f * ((float)y + jy) / (float)height;
+    f2 lens = g.next_vec2();
+    float time = g.next_f32();
+    f3 o, d;
+    camera_ray(*cam, ndc, lens, &o, &d);
+    // a batch ray carries its job in the origin's w (the traversal's t_min is a constant)
+    __stcs(&P.ray_o[0][i], make_float4(o.x, o.y, o.z, BATCH ? __uint_as_float(job) : 1e-4f));
+    __stcs(&P.ray_d[0][i], make_float4(d.x, d.y, d.z, time));
+    store_rng(P.rng, i, g);
+    // radiance 0, throughput 1 and the AOVs are set by shade at depth 0;
+    // with max_depth 0 no vertex is shaded and the sample is all zeros
+    if (max_depth == 0) {
+        P.Lb[2 * (size_t)i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        stcs_256(P.aov + 2 * (size_t)i, make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+    }
+    for (uint32_t s = 0; s < W.ns; ++s) __stcs(P.pend + (size_t)i * W.ns + s, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+}
 template <bool BATCH>
 __global__ void k_raygen(PathSoA P, WaveParams W) {
     const uint32_t n = P.ctl->n_valid;
     const uint32_t s_base = P.ctl->s_base, kv = P.ctl->k_valid;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t x, y, s, width, height, max_depth = W.max_depth, job = 0;
-        const DevCamera* cam = &W.cam;
-        if (BATCH) {
-            const DevWave& wv = W.waves[P.ctl->wave];
-            const DevSeg sg = W.segs[find_segment(W.segs, wv, i, false)];
-            const DevJob& J = W.jobs[sg.job];
-            const TilePixel t = tile_pixel(J.width, J.height, sg.s_count, i - sg.path_base);
-            x = t.x; y = t.y; s = sg.s_first + t.k;
-            width = J.width; height = J.height;
-            max_depth = J.max_depth;
-            cam = &J.cam;
-            job = sg.job;
-        } else {
-            const TilePixel t = tile_pixel(W.cw, W.ch, kv, i);
-            x = W.cx0 + t.x; y = W.cy0 + t.y; s = s_base + t.k;
-            width = W.width; height = W.height;
-        }
-        Rng g;
-        g.seed(pixel_seed(x, y, s));
-        float jx = g.next_f32(), jy = g.next_f32();
-        f2 ndc;
-        ndc.x = 2.0f * ((float)x + jx) / (float)width - 1.0f;
-        ndc.y = 1.0f - 2.0f * ((float)y + jy) / (float)height;
-        f2 lens = g.next_vec2();
-        float time = g.next_f32();
-        f3 o, d;
-        camera_ray(*cam, ndc, lens, &o, &d);
-        // a batch ray carries its job in the origin's w (the traversal's t_min is a constant)
-        __stcs(&P.ray_o[0][i], make_float4(o.x, o.y, o.z, BATCH ? __uint_as_float(job) : 1e-4f));
-        __stcs(&P.ray_d[0][i], make_float4(d.x, d.y, d.z, time));
-        store_rng(P.rng, i, g);
-        // radiance 0, throughput 1 and the AOVs are set by shade at depth 0;
-        // with max_depth 0 no vertex is shaded and the sample is all zeros
-        if (max_depth == 0) {
-            P.Lb[2 * (size_t)i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            stcs_256(P.aov + 2 * (size_t)i, make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-        }
-        for (uint32_t s = 0; s < W.ns; ++s) __stcs(P.pend + (size_t)i * W.ns + s, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        raygen_path<BATCH>(P, W, s_base, kv, i);
 }
 
 // ---------------------------------------------------------------- extend --
@@ -363,8 +367,10 @@ struct ExtendRays {
     const PathSoA* P;
     const WaveParams* W;
     uint32_t depth;
-    // ray p of the queue sits at queue position p (depth 0: path p)
-    __device__ __forceinline__ uint32_t load(uint32_t p, TraceRay& r, int32_t& root) const {
+    uint32_t base = 0;  // first queue position
+    // ray j of the queue sits at queue position base + j (depth 0: that path)
+    __device__ __forceinline__ uint32_t load(uint32_t j, TraceRay& r, int32_t& root) const {
+        const uint32_t p = base + j;
         const float4 ro = __ldcs(P->ray_o[depth & 1] + p), rd = __ldcs(P->ray_d[depth & 1] + p);
         r.o = mk3(ro.x, ro.y, ro.z);
         r.d = mk3(rd.x, rd.y, rd.z);
@@ -407,7 +413,9 @@ struct ShadowRays {
     const DevScene* S;
     const PathSoA* P;
     const WaveParams* W;
+    uint32_t base = 0;  // first queue position
     __device__ __forceinline__ uint32_t load(uint32_t j, TraceRay& r, int32_t& root) const {
+        j += base;
         // the ray sits at its queue entry, so these loads do not wait for sq
         const uint32_t target = __ldcs(P->sq + j);
         const float4 so = __ldcs(P->sh_o + j), sd = __ldcs(P->sh_d + j);
@@ -433,6 +441,24 @@ __global__ void __launch_bounds__(128, PYRE_SHADOW_BLOCKS(WIDTH)) k_shadow(DevSc
     trace_stream<true, WIDTH>(S, src, P.ctl->scount[depth], &P.ctl->fetch[2 * depth + 1], W.refill_any);
 }
 
+// Shadow rays and extend rays by one team of warps.
+template <class SrcS, class SrcE>
+__device__ __forceinline__ void trace_both(const DevScene& S, const SrcS& shadow, uint32_t ns, uint32_t* fetch_s, int refill_s,
+                                           const SrcE& extend, uint32_t ne, uint32_t* fetch_e, int refill_e,
+                                           const TraceTeam& all, TraceShared<false>& sh) {
+    TraceTeam t = all, u = all;
+    t.deal = u.deal = (uint64_t)ns + ne < 32u * (uint64_t)all.warps;
+    bool do_extend = true, do_shadow = true;
+    if (t.deal && ne && ns) {  // each queue gets its part of the warps
+        t.warps = max(1u, min(all.warps - 1u, (uint32_t)((uint64_t)all.warps * ne / ((uint64_t)ne + ns))));
+        do_extend = all.warp < t.warps;
+        do_shadow = !do_extend;
+        u.warp = all.warp - t.warps; u.warps = all.warps - t.warps;
+    }
+    if (do_shadow) trace_binary<true>(S, shadow, ns, fetch_s, refill_s, u, sh.stack, sh.ray, sh.hit);
+    if (do_extend) trace_binary<false>(S, extend, ne, fetch_e, refill_e, t, sh.stack, sh.ray, sh.hit);
+}
+
 // The shadow rays of a depth and the extend rays of the next one depend on
 // nothing but the shade between them, and one launch traces both: warps that
 // find the shadow queue empty go on with extend rays, so only one of the two
@@ -445,27 +471,11 @@ __global__ void __launch_bounds__(128, PYRE_SHADOW_BLOCKS(WIDTH)) k_shadow(DevSc
 template <bool BATCH>
 __global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_trace(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     __shared__ TraceShared<false> sh;
-    const uint32_t ns = P.ctl->scount[depth], ne = P.ctl->count[depth + 1];
-    TraceTeam t = whole_grid(0), u = t;
-    t.deal = u.deal = (uint64_t)ns + ne < 32u * (uint64_t)t.warps;
-    bool extend = true, shadow = true;
-    if (t.deal && ne && ns) {
-        // neighbouring warps of the team sit on different SMs
-        const uint32_t w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-        const uint32_t we = max(1u, min(t.warps - 1u, (uint32_t)((uint64_t)t.warps * ne / ((uint64_t)ne + ns))));
-        extend = w < we;
-        shadow = !extend;
-        t.warp = w; t.warps = we;
-        u.warp = w - we; u.warps = u.warps - we;
-    }
-    if (shadow) {
-        ShadowRays<BATCH> src{&S, &P, &W};
-        trace_binary<true>(S, src, ns, &P.ctl->fetch[2 * depth + 1], W.refill_any, u, sh.stack, sh.ray, sh.hit);
-    }
-    if (extend) {
-        ExtendRays<BATCH> src{&S, &P, &W, depth + 1};
-        trace_binary<false>(S, src, ne, &P.ctl->fetch[2 * (depth + 1)], W.refill, t, sh.stack, sh.ray, sh.hit);
-    }
+    // neighbouring warps of the team sit on different SMs
+    const TraceTeam all{(threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (blockDim.x >> 5), false};
+    trace_both(S, ShadowRays<BATCH>{&S, &P, &W}, P.ctl->scount[depth], &P.ctl->fetch[2 * depth + 1], W.refill_any,
+               ExtendRays<BATCH>{&S, &P, &W, depth + 1}, P.ctl->count[depth + 1], &P.ctl->fetch[2 * (depth + 1)], W.refill,
+               all, sh);
 }
 
 // ------------------------------------------------------- adjoint helpers --
@@ -648,22 +658,21 @@ __global__ void __launch_bounds__(256) k_sort_tile(DevScene S, PathSoA P, uint32
 #define SHADE_ENV 2
 constexpr int shade_threads(int lights) { return lights == SHADE_QUADS ? 256 : 224; }
 constexpr int shade_blocks(int lights) { return lights == SHADE_QUADS ? 3 : 4; }
-template <bool BATCH, bool ADJ, int LIGHTS>
-__global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : shade_blocks(LIGHTS))
-    k_shade(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+// shade_queue visits queue entries j, j + stride, ... of n; with SLICE the queues
+// are the part of the wave's from position `base` (shadow queue: base * ns), in
+// no order.
+template <bool BATCH, bool ADJ, int LIGHTS, bool SLICE>
+__device__ __forceinline__ void shade_queue(const DevScene& S, const PathSoA& P, const WaveParams& W, uint32_t depth,
+                                            GradSmem& G, uint32_t j, uint32_t stride, uint32_t n, uint32_t base,
+                                            uint32_t* next_count, uint32_t* shadow_count) {
     constexpr bool QUADS = (LIGHTS & SHADE_QUADS) != 0, ENV = (LIGHTS & SHADE_ENV) != 0;
-    GradSmem G{nullptr, nullptr, nullptr};
-    if (ADJ) G = grad_smem_begin(W.env_cache != 0, W.smem_grad != 0, W.n_mat);
-    const uint32_t n = P.ctl->count[depth];
     const uint32_t* qin = P.q[depth & 1];
     uint32_t* qout = P.q[(depth + 1) & 1];
-    uint32_t* next_count = &P.ctl->count[depth + 1];
-    uint32_t* shadow_count = &P.ctl->scount[depth];
     const bool last_was_specular = depth == 0;  // no specular BSDFs: only camera rays
     const float INF = __int_as_float(0x7f800000);
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    for (; j < n; j += stride) {
         // queue position of the path's ray and hit (depth 0: the path index), and the path
-        const uint32_t pos = W.sort ? P.qsort[j] : j;
+        const uint32_t pos = SLICE ? base + j : W.sort ? P.qsort[j] : j;
         const uint32_t i = depth > 0 ? __ldcs(qin + pos) : pos;
         // a batch ray carries its job in the origin's w
         float4 ro_b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -853,7 +862,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : s
                             // position in the next depth's queue
                             if (depth + 1 < (BATCH ? JB->max_depth : W.max_depth)) {
                                 const f3 nd = to_world(fr, wi);
-                                const uint32_t q = append_slot(next_count);
+                                const uint32_t q = (SLICE ? base : 0u) + append_slot(next_count);
                                 qout[q] = i;
                                 __stcs(P.ray_o[(depth + 1) & 1] + q,
                                        make_float4(p_off.x, p_off.y, p_off.z, BATCH ? ro.w : 1e-4f));
@@ -894,7 +903,7 @@ __global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : s
                         G[1] = make_float4(gm[4], gm[5], __uint_as_float(I.material), 1.0f);
                     }
                     if (sh_ray) {
-                        const uint32_t q = append_slot(shadow_count);
+                        const uint32_t q = (SLICE ? base * W.ns : 0u) + append_slot(shadow_count);
                         __stcs(P.sh_o + q, make_float4(p_off.x, p_off.y, p_off.z, sh_tmax));
                         __stcs(P.sh_d + q, make_float4(sh_dir.x, sh_dir.y, sh_dir.z, time));
                         P.sq[q] = (uint32_t)sidx;
@@ -907,7 +916,65 @@ __global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : s
         // a path without a next ray is not read again, whatever its throughput
         stcs_256(P.Lb + 2 * (size_t)i, make_float4(L.x, L.y, L.z, 0.0f), make_float4(beta.x, beta.y, beta.z, next_pdf));
     }
+}
+
+template <bool BATCH, bool ADJ, int LIGHTS>
+__global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : shade_blocks(LIGHTS))
+    k_shade(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+    GradSmem G{nullptr, nullptr, nullptr};
+    if (ADJ) G = grad_smem_begin(W.env_cache != 0, W.smem_grad != 0, W.n_mat);
+    shade_queue<BATCH, ADJ, LIGHTS, false>(S, P, W, depth, G, blockIdx.x * blockDim.x + threadIdx.x,
+                                           gridDim.x * blockDim.x, P.ctl->count[depth], 0u, &P.ctl->count[depth + 1],
+                                           &P.ctl->scount[depth]);
     if (ADJ) grad_smem_end(G, W.env_grad, W.mat_grad, W.n_mat);  // one atomic per parameter / texel per block
+}
+
+// A small wave in one launch: each block takes a slice of the paths through all
+// its depths, from the camera ray to the last vertex, with the queues of its
+// slice in the wave's arrays and their counts in shared memory. The same
+// stages as the kernels above, in their order, so the results are the same
+// bits. A stage launch costs a few us and as much again until the last of its
+// rays is done, with cold L1s, and a render has over twenty: 0.114 against 0.224
+// ms for 16 k paths of the Cornell box, 0.32 against 0.45 for 77 k of the studio
+// preset, one depth of 8 taking some 12 us.
+// W.sort is not used (results do not depend on the order).
+template <int LIGHTS>
+__global__ void __launch_bounds__(128, 5) k_wave_small(DevScene S, PathSoA P, WaveParams W, uint32_t slice) {
+    __shared__ TraceShared<false> sh;
+    __shared__ uint32_t next, shadow, fetch_e, fetch_s;
+    const uint32_t base = blockIdx.x * slice, n_valid = P.ctl->n_valid;
+    if (base >= n_valid) return;
+    uint32_t n = min(slice, n_valid - base);
+    const uint32_t s_base = P.ctl->s_base, kv = P.ctl->k_valid;
+    const TraceTeam all{threadIdx.x >> 5, blockDim.x >> 5, false};
+    GradSmem G{nullptr, nullptr, nullptr};
+    for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) raygen_path<false>(P, W, s_base, kv, base + j);
+    if (threadIdx.x == 0) { fetch_e = 0; fetch_s = 0; }
+    __syncthreads();
+    {
+        TraceTeam t = all;
+        t.deal = n < 32u * t.warps;
+        trace_binary<false>(S, ExtendRays<false>{&S, &P, &W, 0u, base}, n, &fetch_e, W.refill, t, sh.stack, sh.ray, sh.hit);
+    }
+    unsigned long long rays_e = 0, rays_s = 0;  // counted by every thread, added by one
+    for (uint32_t depth = 0; depth < W.max_depth; ++depth) {
+        __syncthreads();
+        if (threadIdx.x == 0) { next = 0; shadow = 0; fetch_e = 0; fetch_s = 0; }
+        __syncthreads();
+        shade_queue<false, false, LIGHTS, true>(S, P, W, depth, G, threadIdx.x, blockDim.x, n, base, &next, &shadow);
+        __syncthreads();
+        const uint32_t ns = shadow;
+        n = next;
+        rays_e += n; rays_s += ns;
+        if (n == 0 && ns == 0) break;
+        trace_both(S, ShadowRays<false>{&S, &P, &W, base * W.ns}, ns, &fetch_s, W.refill_any,
+                   ExtendRays<false>{&S, &P, &W, depth + 1, base}, n, &fetch_e, W.refill, all, sh);
+        if (n == 0) break;
+    }
+    if (threadIdx.x == 0) {  // k_wave_end adds the camera rays
+        if (rays_e) atomicAdd(&P.ctl->extend_rays, rays_e);
+        if (rays_s) atomicAdd(&P.ctl->shadow_rays, rays_s);
+    }
 }
 
 // Adjoint replay: parked gradient terms of the paths' last vertices.
@@ -1153,6 +1220,7 @@ struct Launch {
     int block_stage = 256;  // raygen, accumulate, adjoint shade (at most 256)
     int block_shade = 0;    // forward shade (at most shade_threads of the scene's lights)
     int lights = SHADE_QUADS;  // the forward shade's LIGHTS
+    int blocks_small = 0;      // resident blocks of k_wave_small; 0: waves run stage by stage
     int block_trace = 128;  // extend, shadow (at most 128)
     int grid_raygen, grid_shade, grid_extend, grid_shadow, grid_trace, grid_acc, grid_sort;
 };
@@ -1193,6 +1261,8 @@ Launch make_launch(pyre_ctx* ctx, const DevScene& S, uint32_t block_size, int wi
                     : width == 4 ? grid_for(ctx, k_shadow<BATCH, 4>, L.block_trace)
                                  : grid_for(ctx, k_shadow<BATCH, 2>, L.block_trace);
     L.grid_trace = grid_for(ctx, k_trace<BATCH>, L.block_trace);
+    if (!BATCH && !block_size && width == 2)
+        with_lights<false>(L.lights, [&](auto l) { L.blocks_small = grid_for(ctx, k_wave_small<l()>, 128); });
     L.grid_acc = BATCH ? grid_for(ctx, k_accumulate_batch, L.block_stage) : grid_for(ctx, k_accumulate, L.block_stage);
     L.grid_sort = grid_for(ctx, k_sort_scatter, 256);
     return L;
@@ -1267,11 +1337,35 @@ void enqueue_sort(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const Laun
     k_sort_scatter<<<Lc.grid_sort, 256, 0, st>>>(S, P, d);
 }
 
+// Waves of up to this many paths run as one launch (k_wave_small): 131 k paths of
+// the Cornell box 0.194 against 0.264 ms, 120 k of the Cornell preset 0.42
+// against 0.49, 77 k of the procedural studio 0.60 against 0.77; 173 k of the
+// studio preset took 0.504 either way, 262 k of the Cornell box 0.322 against
+// 0.367, 307 k of the procedural studio 1.31 against 1.07: with more rays than the
+// launch holds at once, its stages at 5 blocks per SM lose to the stage kernels'
+// 9 and 10.
+#define PYRE_SMALL_WAVE (128u << 10)
+bool small_wave(const pyre_ctx* ctx, const WaveParams& W, const Launch& Lc) {
+    return Lc.blocks_small && !ctx->stage_timing && W.max_depth > 0 &&
+           (uint64_t)W.npix * W.k_per_wave <= PYRE_SMALL_WAVE;
+}
+
 void enqueue_wave(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, const WaveParams& W, const Launch& Lc,
                   DeviceStatus* status) {
     cudaStream_t st = ctx->stream;
     mark(ctx, STAGE_OTHER);
     k_wave_begin<<<1, 32, 0, st>>>(P.ctl, W.spp_begin, W.spp_end, W.k_per_wave, W.npix);
+    if (small_wave(ctx, W, Lc)) {
+        const uint32_t paths = W.npix * W.k_per_wave;
+        uint32_t slice = (paths + Lc.blocks_small - 1) / Lc.blocks_small;
+        slice = std::max(32u, (slice + 31) / 32 * 32);
+        with_lights<false>(Lc.lights, [&](auto l) {
+            k_wave_small<l()><<<(paths + slice - 1) / slice, 128, 0, st>>>(S, P, W, slice);
+        });
+        k_accumulate<<<Lc.grid_acc, Lc.block_stage, 0, st>>>(P, W);
+        k_wave_end<<<1, 32, 0, st>>>(P.ctl, W.max_depth, S.error_flag, status);
+        return;
+    }
     k_raygen<false><<<Lc.grid_raygen, Lc.block_stage, 0, st>>>(P, W);
     mark(ctx, STAGE_EXTEND);
     if (W.max_depth) launch_extend<false>(st, Lc, S, P, W, 0);
@@ -1308,8 +1402,8 @@ void enqueue_wave_batch(pyre_ctx* ctx, const DevScene& S, const PathSoA& P, cons
     mark(ctx, STAGE_END);
 }
 
-uint32_t kernels_per_wave(const pyre_ctx* ctx, const WaveParams& W) {
-    if (W.max_depth == 0) return 4;
+uint32_t kernels_per_wave(const pyre_ctx* ctx, const WaveParams& W, bool small = false) {
+    if (small || W.max_depth == 0) return 4;
     const uint32_t sorts = W.sort == PYRE_SORT_TILES ? 1 : W.sort ? 3 : 0;
     // extend at depth 0, then per depth the sorts, shade, the shadow rays and the next depth's extend rays
     const uint32_t traces = W.ns == 0 ? W.max_depth : one_trace_launch(ctx, W) ? W.max_depth + 1 : 2 * W.max_depth;
@@ -1525,7 +1619,7 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
     if (staged)
         for (int c = 0; c < 4; ++c)
             if (out[c]) std::memcpy(out[c], ctx->h_stage + offs[c] * sizeof(float), channel_bytes(c));
-    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W) + 1);
+    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W, small_wave(ctx, W, Lc)) + 1);
     pyre_render_stats& s = ctx->stats;
     if (ctx->stage_timing) {
         float acc[4] = {0, 0, 0, 0};
@@ -1863,7 +1957,7 @@ extern "C" int pyre_render_noalloc(pyre_ctx* ctx, const pyre_scene* scene, const
     DeviceStatus ds;
     if ((rc = read_back(ctx, (const char*)ctx->d_status, 0, &ds))) return rc;
     if ((rc = kernel_error(ctx, ds.error))) return rc;
-    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W) + 1);
+    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W, small_wave(ctx, W, Lc)) + 1);
     return PYRE_OK;
 }
 
