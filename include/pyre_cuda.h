@@ -264,7 +264,7 @@ typedef struct pyre_render_params {
     uint32_t wave_paths;             /* paths in flight per wave; 0 = automatic (what a quarter
                                         of the free device memory holds, 8 Mi to 128 Mi) */
     uint32_t block_size;             /* threads per block of the stage kernels (at most 256;
-                                        224 for the forward shade of a scene with an
+                                        192 for the forward shade of a scene with an
                                         environment, 128 for the traversals);
                                         0 = those */
     uint32_t sort_by_material;       /* order the shade queue by material: 1 = within

@@ -1,7 +1,7 @@
 """Autotuner for the wavefront's launch knobs.
 
 Knobs (pyre_render_params): wave_paths (queue capacity = paths in flight per
-wave), block_size (threads per block of the stage kernels, capped at 224 for
+wave), block_size (threads per block of the stage kernels, capped at 192 for
 the forward shade of a scene with an environment and at 128 for the
 traversals; 0 = those, 256 elsewhere), use_graph (CUDA-graph replay),
 sort_by_material (shade visits the live paths sorted by material) and

@@ -128,10 +128,9 @@ struct TraceHit {
 #define PYRE_STEPS_PER_VOTE 6
 #endif
 
-// 32 B with one load (sm_100+; p is 32-B aligned). A traversal step fetches
-// its 64-B node with two of these instead of four 128-bit loads: 763.4 against
-// 749.8 Msamples/s on the 1080p studio frame, the traversal being bound by
-// instruction issue.
+// 32 B with one load (sm_100+; p is 32-B aligned): half the load instructions
+// of 128-bit ones, and of the L1's data cycles where every lane reads a record of
+// its own (46.4 against 77.3 cycles per 64-B record of 32 lanes).
 __device__ __forceinline__ void ldg_256(const float4* p, float4& a, float4& b) {
     asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)

@@ -113,8 +113,8 @@ struct WaveParams {
 // Default ray-refill thresholds (idle lanes of a warp) of closest-hit and
 // any-hit traversal; a nonzero refill_lanes sets both. Closest hit at 12
 // (with lanes that stop at their first leaf and the leaf phase at 16 seeking
-// lanes): 762.3 against 758.8 Msamples/s for 16 and 755.2 for 20 on the
-// 1080p studio frame; microbenchmark closest hit 3.75 against 4.01 ms.
+// lanes): 8 and 16 are within half a per cent of it on the 1080p studio frame
+// and the closest-hit queries.
 #ifndef PYRE_DEFAULT_REFILL
 #define PYRE_DEFAULT_REFILL 12
 #endif
@@ -359,8 +359,7 @@ __global__ void k_raygen(PathSoA P, WaveParams W) {
 template <bool BATCH>
 struct ExtendRays {
     // every extend ray has this t range (the traversal's idle lanes start
-    // with it too, so the compiler keeps it out of registers: spills 16
-    // against 28 B, 811.4 against 802.4 Msamples/s on the 1080p studio frame)
+    // with it too, so the compiler keeps it out of registers)
     static constexpr float kTmin = 1e-4f, kTmax = INFINITY;
     static constexpr bool kFixedTmin = true;
     const DevScene* S;
@@ -647,17 +646,26 @@ __global__ void __launch_bounds__(256) k_sort_tile(DevScene S, PathSoA P, uint32
 // environment its code is left out, which a kernel this large pays for in
 // registers and instruction fetches: 2.05 against 2.19 ms of shade on the Cornell
 // preset at 800x600 and 16 spp, 213 against 215 ms on a batch of 40 views.
-// Threads and resident blocks: bound by load latency, 24 to 28 warps per SM.
-// Quad lights only: 256 x 3 (80 registers), 128 x 6 / 192 x 4 the same, 224 x 4
-// 2.19 against 2.05 ms and 236 against 213 ms on the batch. With an environment:
-// 224 x 4 (72 registers) 35.6 ms per 1080p studio frame, 256 x 3 36.6, 192 x 5 and
-// 128 x 8 37.9 and 42.5 (before the material terms below). The adjoint keeps 3
-// blocks of 256; leaving out the quad lights there gave 14.9 against 15.2 ms of
-// backward on the 512^2 problem (the forward lost 1 ms of 35.6 that way).
+// Threads and resident blocks: bound by load latency, 24 to 30 warps per SM.
+// Quad lights only: 256 x 3 (80 registers) 1.91 ms on the Cornell preset and 203 ms
+// on the batch, 224 x 4 1.94 and 204, 256 x 4 1.92 and 217, 192 x 5 1.95 and 216.
+// With an environment: 192 x 5 (64 registers) 30.6 ms of shade per 1080p studio frame
+// and 0.51 on a 959x541 one, 224 x 4 32.3 and 0.51, 224 x 5 30.9 and 0.50 (but 0.176
+// against 0.167 on a viewer's pass), 128 x 7 32.4, 256 x 4 34.8, 256 x 3 34.5. The
+// adjoint keeps 3 blocks of 256; leaving out the quad lights there gave 14.9 against
+// 15.2 ms of backward on the 512^2 problem (the forward lost by it).
+//
+// Registers that do not fit spill to shared memory (a PTX pragma; kernels with
+// dynamic shared memory, as the adjoint, cannot use it). In local memory they
+// shared the L1 with the path state that streams through it, which hits 21 to 30 %
+// of the time, so that most reloads went to L2: 32.3 against 34.5 ms per 1080p studio
+// frame at 224 x 4, 202.6 against 209.8 ms on the batch, 1.91 against 2.00 on the
+// Cornell preset.
+#define PYRE_SPILL_TO_SMEM asm volatile(".pragma \"enable_smem_spilling\";")
 #define SHADE_QUADS 1
 #define SHADE_ENV 2
-constexpr int shade_threads(int lights) { return lights == SHADE_QUADS ? 256 : 224; }
-constexpr int shade_blocks(int lights) { return lights == SHADE_QUADS ? 3 : 4; }
+constexpr int shade_threads(int lights) { return lights == SHADE_QUADS ? 256 : 192; }
+constexpr int shade_blocks(int lights) { return lights == SHADE_QUADS ? 3 : 5; }
 // shade_queue visits queue entries j, j + stride, ... of n; with SLICE the queues
 // are the part of the wave's from position `base` (shadow queue: base * ns), in
 // no order.
@@ -925,8 +933,9 @@ __device__ __forceinline__ void shade_queue(const DevScene& S, const PathSoA& P,
 template <bool BATCH, bool ADJ, int LIGHTS>
 __global__ void __launch_bounds__(ADJ ? 256 : shade_threads(LIGHTS), ADJ ? 3 : shade_blocks(LIGHTS))
     k_shade(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+    if constexpr (!ADJ) PYRE_SPILL_TO_SMEM;
     GradSmem G{nullptr, nullptr, nullptr};
-    if (ADJ) G = grad_smem_begin(W.env_cache != 0, W.smem_grad != 0, W.n_mat);
+    if constexpr (ADJ) G = grad_smem_begin(W.env_cache != 0, W.smem_grad != 0, W.n_mat);
     shade_queue<BATCH, ADJ, LIGHTS, false>(S, P, W, depth, G, blockIdx.x * blockDim.x + threadIdx.x,
                                            gridDim.x * blockDim.x, P.ctl->count[depth], 0u, &P.ctl->count[depth + 1],
                                            &P.ctl->scount[depth]);
