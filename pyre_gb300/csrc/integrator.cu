@@ -393,7 +393,7 @@ struct ExtendRays {
 };
 
 // The traversal kernels are persistent grids of resident 128-thread blocks,
-// 9 or 10 per SM (56 or 48 registers). Warps wait mostly on node, triangle and stack
+// 9 or 10 per SM (56 or 48 registers). Warps wait mostly on node and triangle
 // loads, so more of them per SM pay, up to where the spills that a smaller
 // register budget forces cost more than the extra warps hide.
 template <bool BATCH, int WIDTH>
@@ -572,19 +572,17 @@ __global__ void k_sort_scatter(DevScene S, PathSoA P, uint32_t depth) {
 // one block sorts a tile by shade key in shared memory (a warp-aggregated
 // histogram, a block scan, a scatter) and writes the tile's part of P.qsort.
 // Shade's warps mostly see one material at a time, while its path-state reads
-// stay within the tile. On the 1080p studio frame (65 materials, Disney BSDFs,
-// environment NEE), with tiles of 2048 entries: 781.2 against 770.9
-// Msamples/s unsorted (shade 41.5 against 43.3 ms, and the next extend 91.7
-// against 92.0); sorting the whole queue gave 733.6. On the Cornell views of the batch workload (Lambertian
-// walls, quad-light NEE) shade is bound by its path-state traffic, and the
-// sorted order, which spreads a warp's path indices over the tile, doubles
-// its time at bounces 1-3 (9.3 against 5.0 ms at bounce 1 of a 1024^2 view at
-// 64 spp). Rendering therefore leaves the queue unsorted unless asked.
+// stay within the tile. The 1080p studio frame (65 materials, Disney BSDFs,
+// environment NEE) takes 115.0 ms sorted within tiles, 116.7 unsorted and 132.5 with
+// the whole queue sorted. On Cornell views (Lambertian walls, quad-light NEE) shade
+// is bound by its path-state traffic, and the sorted order spreads a warp's path
+// indices over the tile: the Cornell preset at 800x600 6.50 against 5.71 ms, a batch
+// of 40 views 263 against 213. Rendering therefore leaves the queue unsorted unless
+// asked.
 // Within a tile, paths of one key land in any order; shade's results do not
 // depend on the order in which it visits paths.
 // Queue entries per tile, PYRE_SORT_TILE_E per thread of a 256-thread block:
-// on the 1080p studio frame 1024 / 2048 / 4096 / 8192 / 16384 entries gave
-// 766.5 / 784.2 / 793.4 / 791.0 / 782.4 Msamples/s.
+// 2048 / 4096 / 8192 gave 36.7 / 35.6 / 36.1 ms of sort and shade per 1080p studio frame.
 #ifndef PYRE_SORT_TILE_N
 #define PYRE_SORT_TILE_N 4096
 #endif
@@ -1212,8 +1210,8 @@ size_t carve_paths(char* base, size_t P, uint32_t ns, uint32_t npix, PathSoA* ou
 
 // Default wave capacity: the paths whose state fits a quarter of the device
 // memory that is free (counting this context's own path workspace), between
-// 8 Mi and 128 Mi paths. On the 1080p 64-spp studio frame 8, 16, 32, 64 and
-// 128 Mi paths gave 444, 479, 497, 506 and 510 Msamples/s: the last bounces
+// 8 Mi and 128 Mi paths. The 1080p 64-spp studio frame takes 133.3, 124.6,
+// 118.9, 116.3 and 115.0 ms with 8, 16, 32, 64 and 128 Mi paths: the last bounces
 // of a wave hold few live paths, and a larger wave spends a smaller share of
 // those launches draining the warps' final rays. A call of at most 8 Mi paths
 // (all) fits any of these and does not ask for the free memory.
@@ -2195,8 +2193,8 @@ extern "C" int pyre_backward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_
     // The adjoint shade is bound by instruction fetches: warps of one
     // material run one branch of the BSDF and gradient code. Sorting the
     // whole live-path queue by material is the backward's default: backward
-    // 20.0 against 22.2 ms on the 512x512 differentiable-render problem, the
-    // same gradients; sorting within tiles (the render default) gave 20.5.
+    // 14.0 against 14.8 ms on the 512x512 differentiable-render problem, the
+    // same gradients; sorting within tiles gave 14.1.
     W.sort = sort_kind(rp.sort_by_material, PYRE_SORT_QUEUE);
     if (W.sort < 0) return set_error(ctx, PYRE_ERR_INVALID, "sort_by_material must be 0, 1, 2 or 3");
     DevScene D;
