@@ -698,7 +698,7 @@ def main():
         roofline["traffic"] = tj.get("bytes_per_launch")
         roofline["traffic_note"] = tj.get("note")
     counters_file = ROOT / "profiles" / "k_extend_counters.json"
-    if counters_file.exists():  # the kernel is issue-bound: these counters say more than the HBM fraction
+    if counters_file.exists():  # bound by L1 data cycles and load latency: these counters say more than the HBM fraction
         roofline["ncu_counters_bounces_0_1_2"] = json.loads(counters_file.read_text())
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
