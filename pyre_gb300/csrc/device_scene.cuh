@@ -138,11 +138,13 @@ __device__ __forceinline__ void ldg_256(const float4* p, float4& a, float4& b) {
 }
 
 // 32-B path-state records with one streaming (evict-first) 256-bit load or
-// store each; p must be 32-B aligned.
+// store each; p must be 32-B aligned. The load stays where it is among the
+// stores and barriers: k_wave_small reads back what it wrote a depth before.
 __device__ __forceinline__ void ldcs_256(const float4* p, float4& a, float4& b) {
-    asm("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
+    asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
 }
 __device__ __forceinline__ void stcs_256(float4* p, const float4& a, const float4& b) {
     asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
