@@ -1422,6 +1422,19 @@ uint32_t kernels_per_wave(const pyre_ctx* ctx, const WaveParams& W, bool small =
     return 4 + W.max_depth * (sorts + 1) + traces;
 }
 
+// Names a captured wave: the kernels it launches (W, Lc) and every argument that
+// they got by value. All of it is plain data.
+std::string graph_key(const char* kind, const pyre_scene* scene, const DevScene& D, const PathSoA& S,
+                      const WaveParams& W, const Launch& Lc) {
+    std::string k = std::string(kind) + "/" + std::to_string(scene->serial) + "/";
+    auto add = [&](const auto& v) {
+        static_assert(std::is_trivially_copyable_v<std::remove_reference_t<decltype(v)>>, "bytes of a plain struct");
+        k.append(reinterpret_cast<const char*>(&v), sizeof v);
+    };
+    add(D); add(S); add(W); add(Lc);
+    return k;
+}
+
 // Clears the film sums and the wave counters: consecutive arrays (carve_paths), one memset.
 int clear_sums(pyre_ctx* ctx, const PathSoA& S) {
     const size_t bytes = (size_t)((const char*)(S.ctl + 1) - (const char*)S.acc_r);
@@ -1585,17 +1598,8 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
     DeviceStatus* d_status = staged ? (DeviceStatus*)((char*)staging + film_bytes) : ctx->d_status;
     if (graph) {
         // One wave captured once per configuration, replayed `waves` times.
-        char key[256];
-        std::snprintf(key, sizeof key, "%llu/%p/%u/%u/%u/%u/%u/%u/%u/%u/%d/r%d/s%d/w%d",
-                      (unsigned long long)scene->serial, ctx->render_ws.ptr, W.npix, W.k_per_wave, W.max_depth,
-                      W.min_rr, W.ns, W.spp_begin, W.spp_end, W.cx0 + W.cy0 * 65536u, W.env_cdf, W.refill, W.sort,
-                      W.bvh_width);
-        std::string k2 = std::string(key) + "/" + std::to_string(W.width) + "x" + std::to_string(W.height) + "/b" +
-                         std::to_string(Lc.block_stage) + "x" + std::to_string(Lc.block_shade) + "x" +
-                         std::to_string(Lc.block_trace);
-        // camera bytes are part of the key
-        k2.append(reinterpret_cast<const char*>(&W.cam), sizeof(W.cam));
-        if (!ctx->wave_graph || ctx->wave_graph_key != k2) {
+        const std::string key = graph_key("wave", scene, D, S, W, Lc);
+        if (!ctx->wave_graph || ctx->wave_graph_key != key) {
             if (ctx->wave_graph) { cudaGraphExecDestroy(ctx->wave_graph); ctx->wave_graph = nullptr; }
             cudaGraph_t g;
             PYRE_CUDA_TRY(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1604,7 +1608,7 @@ static int render_impl(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera
             cudaError_t e = cudaGraphInstantiate(&ctx->wave_graph, g, 0);
             cudaGraphDestroy(g);
             if (e != cudaSuccess) { ctx->wave_graph = nullptr; return cuda_check(ctx, e, "cudaGraphInstantiate"); }
-            ctx->wave_graph_key = k2;
+            ctx->wave_graph_key = key;
         }
         for (uint32_t w = 0; w < waves; ++w) PYRE_CUDA_TRY(ctx, cudaGraphLaunch(ctx->wave_graph, st));
     } else {
@@ -1796,13 +1800,7 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
         // One wave (its bounce loop) as a graph: every wave runs the same kernels, and the kernels read which
         // segments the current wave holds from the device tables (WaveCtl::wave), so the graph is replayed
         // once per wave.
-        std::string key = "batchwave/" + std::to_string(scene->serial) + "/" +
-                          std::to_string((uintptr_t)ctx->render_ws.ptr) + "/" + std::to_string(max_depth) + "/" +
-                          std::to_string(max_paths) + "/" + std::to_string(total_pix) + "/" +
-                          std::to_string(dj.size()) + "/" + std::to_string(segs.size()) + "/b" +
-                          std::to_string(Lc.block_stage) + "x" + std::to_string(Lc.block_shade) + "x" +
-                          std::to_string(Lc.block_trace) + "/r" + std::to_string(W.refill) + "/s" +
-                          std::to_string(W.sort) + "/w" + std::to_string(W.bvh_width);
+        const std::string key = graph_key("batch", scene, D, S, W, Lc);
         if (!ctx->wave_graph || ctx->wave_graph_key != key) {
             if (ctx->wave_graph) { cudaGraphExecDestroy(ctx->wave_graph); ctx->wave_graph = nullptr; }
             cudaGraph_t g;
