@@ -346,10 +346,10 @@ int pyre_forward(pyre_ctx* ctx, const pyre_scene* scene, const pyre_camera_desc*
  * replays every path of the sample range from its pixel seed, through the same
  * wavefront kernels as the forward, and writes the gradients. It uses the
  * radiance kept by the last pyre_forward with the same scene, camera and
- * params, or renders it first. Convention: detached sampling; only BSDF
- * values and emitted radiance carry derivatives (pdfs, MIS weights, lobe
- * choice, Russian roulette and the environment's sampling tables are
- * constants), which is unbiased for the derivative of the expected image.
+ * params (and no new materials or environment since), or renders it first.
+ * Convention: detached sampling; only BSDF values and emitted radiance carry
+ * derivatives (pdfs, MIS weights, lobe choice, Russian roulette and the
+ * environment's sampling tables are constants), which is unbiased for the derivative of the expected image.
  * Single (non-batch) scenes only. A colour channel whose BSDF value is
  * exactly zero at a vertex loses that vertex's BSDF-sample term in that
  * channel (the replay divides the remaining radiance by f). */

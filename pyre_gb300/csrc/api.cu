@@ -922,6 +922,7 @@ int pyre_scene_set_materials(pyre_ctx* ctx, pyre_scene* scene, const pyre_materi
     }
     cudaSetDevice(ctx->device);
     PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    scene->parameters += 1;  // a kept forward pass saw the old materials
     if (n) PYRE_CUDA_TRY(ctx, cudaMemcpy((void*)scene->dev.materials, mats.data(), n * sizeof(DevMaterial),
                                          cudaMemcpyHostToDevice));
     return PYRE_OK;
@@ -935,6 +936,7 @@ int pyre_scene_set_env(pyre_ctx* ctx, pyre_scene* scene, const float* rgb, float
     build_env_tables(E.width, E.height, rgb, t);
     cudaSetDevice(ctx->device);
     PYRE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    scene->parameters += 1;
     auto put = [&](const void* dst, const void* src, size_t bytes) {
         return cudaMemcpy(const_cast<void*>(dst), src, bytes, cudaMemcpyHostToDevice);
     };

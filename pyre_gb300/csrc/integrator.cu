@@ -2115,7 +2115,7 @@ int pyre_intersect_any(pyre_ctx* ctx, const pyre_scene* scene, const pyre_rays* 
 // sums contributions in the forward's order.
 namespace {
 std::string tape_key(const pyre_scene* scene, const pyre_camera_desc* camera, const pyre_render_params& rp) {
-    std::string k = std::to_string(scene->serial) + "/";
+    std::string k = std::to_string(scene->serial) + "/" + std::to_string(scene->parameters) + "/";
     k.append(reinterpret_cast<const char*>(camera), sizeof *camera);
     const uint32_t f[] = {rp.width, rp.height, rp.spp_begin, rp.spp_end, rp.max_depth, rp.min_rr_depth,
                           rp.crop[0], rp.crop[1], rp.crop[2], rp.crop[3], rp.env_sampling};

@@ -13,6 +13,7 @@
 struct pyre_scene {
     pyre::DevScene dev;
     uint64_t serial = 0;  // unique per upload; keys cached CUDA graphs
+    uint64_t parameters = 0;  // changes with every new set of materials or texels; keys the kept radiance
     std::vector<void*> allocations;  // device buffers owned by the scene
     std::vector<int32_t> slot_of_instance;  // original instance id -> device slot
     uint32_t n_triangles = 0;
