@@ -1958,6 +1958,7 @@ extern "C" int pyre_render_noalloc(pyre_ctx* ctx, const pyre_scene* scene, const
     const int timing = ctx->stage_timing;
     ctx->stage_timing = 0;  // stage timing would create events
     for (uint32_t w = 0; w < waves; ++w) enqueue_wave(ctx, D, S, W, Lc, ctx->d_status);
+    const uint32_t launches = waves * kernels_per_wave(ctx, W, small_wave(ctx, W, Lc)) + 1;
     ctx->stage_timing = timing;
     PYRE_CUDA_TRY(ctx, cudaGetLastError());
     k_finalize<<<Lc.grid_acc, 256, 0, st>>>(S, W.npix, 1.0f / (float)spp, film->radiance, film->albedo, film->normal,
@@ -1967,7 +1968,7 @@ extern "C" int pyre_render_noalloc(pyre_ctx* ctx, const pyre_scene* scene, const
     DeviceStatus ds;
     if ((rc = read_back(ctx, (const char*)ctx->d_status, 0, &ds))) return rc;
     if ((rc = kernel_error(ctx, ds.error))) return rc;
-    fill_stats(ctx, ds, waves, waves * kernels_per_wave(ctx, W, small_wave(ctx, W, Lc)) + 1);
+    fill_stats(ctx, ds, waves, launches);
     return PYRE_OK;
 }
 
