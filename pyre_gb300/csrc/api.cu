@@ -284,9 +284,10 @@ __global__ void k_pack_nodes(GpuNode* __restrict__ nodes, uint32_t n_nodes, uint
                 tris[3 * (size_t)(child + count - 1) + 2].w = __uint_as_float(1u);
             } else {
                 const int32_t k = count > 0 ? child : child & ~(PYRE_TAG_INST | PYRE_TAG_TOP);
-                const bool direct = count < 0 && inst[k].direct;
-                kind[s] = direct ? INTERIOR : ENTRY;
-                ref[s] = direct ? inst[k].blas_root : PYRE_REF_INST | k;
+                const uint32_t hang = inst[k].hang;
+                kind[s] = hang == PYRE_HANG_ENTRY ? ENTRY : INTERIOR;
+                ref[s] = hang == PYRE_HANG_DIRECT ? inst[k].blas_root
+                                                  : (hang == PYRE_HANG_STATIC ? PYRE_REF_STATIC : PYRE_REF_INST) | k;
             }
             f[4 * s] = lo[0]; f[4 * s + 1] = lo[1]; f[4 * s + 2] = hi[0]; f[4 * s + 3] = hi[1];
             f[8 + 2 * s] = lo[2]; f[9 + 2 * s] = hi[2];
@@ -620,12 +621,14 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
         // (bvh.rs:103-110) and the lane then enters the instance without a
         // node step of its own. Where no other instance uses the mesh, the
         // binary traversal has no entry at all (k_pack_nodes).
+        std::vector<char> own_leaf(tp.size(), 0);
         for (size_t g = first_top; g < nodes.size(); ++g)
             for (int c = 0; c < 2; ++c) {
                 if (nodes[g].d[2 + c] != 1) continue;
                 const int32_t slot = nodes[g].d[c];
                 const pyre_instance_desc& id = desc->instances[live[tp[(size_t)(slot - slot_base)]]];
                 if (id.has_motion) continue;
+                own_leaf[(size_t)(slot - slot_base)] = 1;
                 set_gpu_child(nodes[g], c, mesh_box[id.mesh], slot | PYRE_TAG_INST | PYRE_TAG_TOP, -1);
             }
         inst.resize(inst.size() + tp.size());
@@ -643,8 +646,8 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
             I.has_motion = id.has_motion ? 1 : 0;
             for (int c = 0; c < 3; ++c) { I.off0[c] = id.offset_t0[c]; I.off1[c] = id.offset_t1[c]; }
             I.orig_id = (int32_t)i;
-            I.direct = !id.has_motion && mesh_users[id.mesh] == 1 ? 1u : 0u;
-            if (I.direct) mesh_inst[id.mesh] = slot_base + (int32_t)k;
+            if (!id.has_motion && mesh_users[id.mesh] == 1) mesh_inst[id.mesh] = slot_base + (int32_t)k;
+            if (own_leaf[k]) I.hang = mesh_users[id.mesh] == 1 ? PYRE_HANG_DIRECT : PYRE_HANG_STATIC;
             I.material = id.material;
             I.index_base = (uint32_t)mesh_index_base[id.mesh];
             I.normal_base = mesh_normal_base[id.mesh];
