@@ -37,6 +37,21 @@ bool injected_alloc_failure(pyre_ctx* ctx) {
     return false;
 }
 
+cudaError_t device_alloc(pyre_ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->build_ws.ptr && !ctx->building) {
+        cudaFree(ctx->build_ws.ptr);
+        ctx->build_ws = Workspace{};
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();  // an allocation failure is not sticky: clear it for the next launch checks
+    }
+    return e;
+}
+
 int ensure_workspace(pyre_ctx* ctx, Workspace& ws, size_t bytes) {
     if (ws.bytes >= bytes) return PYRE_OK;
     if (ws.ptr) {
@@ -53,12 +68,8 @@ int ensure_workspace(pyre_ctx* ctx, Workspace& ws, size_t bytes) {
     if (injected_alloc_failure(ctx))
         return set_error(ctx, PYRE_ERR_OOM, "cudaMalloc(workspace): injected allocation failure");
     size_t rounded = (bytes + (1u << 20) - 1) & ~(size_t)((1u << 20) - 1);
-    cudaError_t e = cudaMalloc(&ws.ptr, rounded);
-    if (e != cudaSuccess) {
-        ws.ptr = nullptr;
-        cudaGetLastError();  // an allocation failure is not sticky: clear it for the next launch checks
-        return cuda_check(ctx, e, "cudaMalloc(workspace)");
-    }
+    const cudaError_t e = device_alloc(ctx, &ws.ptr, rounded);
+    if (e != cudaSuccess) return cuda_check(ctx, e, "cudaMalloc(workspace)");
     ws.bytes = rounded;
     return PYRE_OK;
 }
@@ -84,11 +95,8 @@ int upload(pyre_ctx* ctx, pyre_scene* sc, const std::vector<T>& host, T** out) {
     size_t bytes = host.size() * sizeof(T);
     if (injected_alloc_failure(ctx))
         return set_error(ctx, PYRE_ERR_OOM, "cudaMalloc(scene): injected allocation failure");
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return cuda_check(ctx, e, "cudaMalloc(scene)");
-    }
+    cudaError_t e = device_alloc(ctx, &p, bytes);
+    if (e != cudaSuccess) return cuda_check(ctx, e, "cudaMalloc(scene)");
     sc->allocations.push_back(p);
     sc->device_bytes += bytes;
     e = cudaMemcpy(p, host.data(), bytes, cudaMemcpyHostToDevice);
@@ -703,7 +711,7 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
     GpuNode* d_nodes = nullptr;
     if (blas.nodes) {  // device-built instance BVHs, then the host-built top levels
         const size_t total = blas.n_nodes + nodes.size();
-        cudaError_t e = cudaMalloc(&d_nodes, total * sizeof(GpuNode));
+        cudaError_t e = device_alloc(ctx, (void**)&d_nodes, total * sizeof(GpuNode));
         if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMalloc(scene)"));
         sc->allocations.push_back(d_nodes);
         sc->device_bytes += total * sizeof(GpuNode);
@@ -757,8 +765,8 @@ static int upload_parts(pyre_ctx* ctx, const pyre_scene_desc* desc, const std::v
         void* p = nullptr;
         if (injected_alloc_failure(ctx))
             return fail(set_error(ctx, PYRE_ERR_OOM, "cudaMalloc(scene): injected allocation failure"));
-        cudaError_t e = cudaMalloc(&p, (size_t)total_tris * 3 * sizeof(float4));
-        if (e != cudaSuccess) { cudaGetLastError(); return fail(cuda_check(ctx, e, "cudaMalloc(scene)")); }
+        cudaError_t e = device_alloc(ctx, &p, (size_t)total_tris * 3 * sizeof(float4));
+        if (e != cudaSuccess) return fail(cuda_check(ctx, e, "cudaMalloc(scene)"));
         sc->allocations.push_back(p);
         sc->device_bytes += (size_t)total_tris * 3 * sizeof(float4);
         const uint32_t grid = (uint32_t)std::min<uint64_t>((total_tris + 255) / 256, 65535);

@@ -73,7 +73,8 @@ struct pyre_ctx {
     Workspace render_ws;        // path state of the wavefront integrator
     Workspace io_ws;            // staging for host-memory rays / films
     Workspace tape_ws;          // pyre_forward: per-path radiance for pyre_backward
-    Workspace build_ws;         // arrays of the GPU BVH build
+    Workspace build_ws;         // arrays of the GPU BVH build, at most 512 MiB between calls
+    bool building = false;      // a build is using them
     Workspace prog_ws;          // pyre_render_progressive: device copy of a host running mean
     int bvh_builder = PYRE_BVH_BUILDER_HOST;  // where pyre_scene_upload builds instance BVHs
     int64_t fail_alloc_countdown = -1;  // pyre_inject_alloc_failure: allocations until one fails
@@ -100,6 +101,8 @@ int set_error(pyre_ctx* ctx, int code, const std::string& msg);
 int cuda_check(pyre_ctx* ctx, cudaError_t e, const char* what);
 // Grows `ws` to at least `bytes` (contents not preserved).
 int ensure_workspace(pyre_ctx* ctx, Workspace& ws, size_t bytes);
+// cudaMalloc; where the device is full, the arrays kept from the last BVH build go first.
+cudaError_t device_alloc(pyre_ctx* ctx, void** p, size_t bytes);
 // True (once) when an injected allocation failure is due (pyre_inject_alloc_failure).
 bool injected_alloc_failure(pyre_ctx* ctx);
 // The status of a kernel error flag read back from the device, which it clears there.
