@@ -131,10 +131,14 @@ struct TraceHit {
 // Node steps a lane takes between two warp votes of the inner phase (a vote, a
 // ballot, a population count and an any, costs issue slots): 3 / 4 / 6 gave
 // 127.5 / 126.9 / 126.6 ms per 1080p studio frame and 2.93 / 2.90 / 2.87 ms on
-// the closest-hit microbenchmark. Films are bit-identical for every setting.
+// the closest-hit microbenchmark. Wide BVHs, whose steps are longer, take 4:
+// the microbenchmark gave 4.33 / 4.35 ms with 4 / 6 at width 4 and 6.21 / 6.32 at
+// width 8, a 960x540 studio frame at 16 spp 14.74 / 14.78 and 19.43 / 19.70.
+// Films are bit-identical for every setting.
 #ifndef PYRE_STEPS_PER_VOTE
 #define PYRE_STEPS_PER_VOTE 6
 #endif
+#define PYRE_STEPS_PER_VOTE_WIDE 4
 
 // 32 B with one load (sm_100+; p is 32-B aligned): half the load instructions
 // of 128-bit ones, and of the L1's data cycles where every lane reads a record of
@@ -745,9 +749,9 @@ __device__ __forceinline__ void trace_wide(const DevScene& S, const Src& src, ui
             const int seeking = __popc(__ballot_sync(FULL, active && !exhausted && !hit_any && parked == 0));
             if (seeking == 0) break;
             if (seeking <= LEAF_WAIT && __any_sync(FULL, active && !hit_any && parked > 0)) break;
-            // each lane takes up to PYRE_STEPS_PER_VOTE node steps between the warp's votes
+            // each lane takes up to PYRE_STEPS_PER_VOTE_WIDE node steps between the warp's votes
 #pragma unroll 1
-            for (int step = 0; step < PYRE_STEPS_PER_VOTE; ++step) {
+            for (int step = 0; step < PYRE_STEPS_PER_VOTE_WIDE; ++step) {
                 if (!active || exhausted || hit_any || parked >= STOP) break;
                 if (node == PYRE_NODE_NONE) {
                     if (sp == 0) { exhausted = true; continue; }
