@@ -268,8 +268,10 @@ typedef struct pyre_render_params {
                                         of the free device memory holds, 8 Mi to 128 Mi) */
     uint32_t block_size;             /* threads per block of the stage kernels (at most 256;
                                         192 for the forward shade of a scene with an
-                                        environment, 128 for the traversals);
-                                        0 = those */
+                                        environment), 0 = those. The traversals always
+                                        take 128. Any other value than 0 also keeps
+                                        small waves (up to 131072 paths) on the stage
+                                        kernels, which take one launch otherwise */
     uint32_t sort_by_material;       /* order the shade queue by material: 1 = within
                                         tiles of 4096 entries, 2 = off, 3 = the whole
                                         queue, 0 = the default (off; 3 in pyre_backward) */

@@ -1,9 +1,9 @@
 """Autotuner for the wavefront's launch knobs.
 
 Knobs (pyre_render_params): wave_paths (queue capacity = paths in flight per
-wave), block_size (threads per block of the stage kernels, capped at 192 for
-the forward shade of a scene with an environment and at 128 for the
-traversals; 0 = those, 256 elsewhere), use_graph (CUDA-graph replay),
+wave), block_size (threads per block of the stage kernels but the traversals,
+capped at 192 for the forward shade of a scene with an environment; 0 = that,
+256 elsewhere, and one launch for a small wave), use_graph (CUDA-graph replay),
 sort_by_material (shade visits the live paths sorted by material) and
 refill_lanes (a warp refetches rays once this many of its lanes are idle) and
 bvh_width (instance BVHs traversed as binary, 4-wide or 8-wide nodes).

@@ -38,6 +38,7 @@ namespace pyre {
 // spills) and shadow 21.7 / 21.7 / 21.4 ms per 1080p studio frame, 1.16 / 1.16 /
 // 1.12 ms on the Cornell preset at 800x600, closest-hit queries 2.68 / 2.53 /
 // 2.56 ms, any hit 0.344 / 0.344 / 0.356 ms. Wide BVHs need more registers.
+#define PYRE_TRACE_THREADS 128
 #define PYRE_TRACE_BLOCKS 9
 #define PYRE_SHADOW_BLOCKS(WIDTH) ((WIDTH) == 2 ? 10 : 9)
 #define PYRE_SORT_BINS 1024  // shade-queue sort keys: escaped, light hit, then materials
@@ -397,7 +398,7 @@ struct ExtendRays {
 // loads, so more of them per SM pay, up to where the spills that a smaller
 // register budget forces cost more than the extra warps hide.
 template <bool BATCH, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_extend(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(PYRE_TRACE_THREADS, PYRE_TRACE_BLOCKS) k_extend(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     ExtendRays<BATCH> src{&S, &P, &W, depth};
     trace_stream<false, WIDTH>(S, src, P.ctl->count[depth], &P.ctl->fetch[2 * depth], W.refill);
 }
@@ -435,7 +436,7 @@ struct ShadowRays {
 };
 
 template <bool BATCH, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_SHADOW_BLOCKS(WIDTH)) k_shadow(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(PYRE_TRACE_THREADS, PYRE_SHADOW_BLOCKS(WIDTH)) k_shadow(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     ShadowRays<BATCH> src{&S, &P, &W};
     trace_stream<true, WIDTH>(S, src, P.ctl->scount[depth], &P.ctl->fetch[2 * depth + 1], W.refill_any);
 }
@@ -468,7 +469,7 @@ __device__ __forceinline__ void trace_both(const DevScene& S, const SrcS& shadow
 // Cornell preset at 800x600 5.69 against 5.81, 1080p studio frame 115.9 against
 // 116.3 (extend rays first: 116.4). Binary BVH only.
 template <bool BATCH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_trace(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
+__global__ void __launch_bounds__(PYRE_TRACE_THREADS, PYRE_TRACE_BLOCKS) k_trace(DevScene S, PathSoA P, WaveParams W, uint32_t depth) {
     __shared__ TraceShared<false> sh;
     // neighbouring warps of the team sit on different SMs
     const TraceTeam all{(threadIdx.x >> 5) * gridDim.x + blockIdx.x, gridDim.x * (blockDim.x >> 5), false};
@@ -1146,7 +1147,7 @@ struct QueryRays {
 };
 
 template <bool ANY, int WIDTH>
-__global__ void __launch_bounds__(128, PYRE_TRACE_BLOCKS) k_intersect(DevScene S, QueryRays q, uint32_t n, unsigned int* counter,
+__global__ void __launch_bounds__(PYRE_TRACE_THREADS, PYRE_TRACE_BLOCKS) k_intersect(DevScene S, QueryRays q, uint32_t n, unsigned int* counter,
                                                    int refill) {
     QueryRays src = q;
     src.S = &S;
@@ -1233,7 +1234,6 @@ struct Launch {
     int block_shade = 0;    // forward shade (at most shade_threads of the scene's lights)
     int lights = SHADE_QUADS;  // the forward shade's LIGHTS
     int blocks_small = 0;      // resident blocks of k_wave_small; 0: waves run stage by stage
-    int block_trace = 128;  // extend, shadow (at most 128)
     int grid_raygen, grid_shade, grid_extend, grid_shadow, grid_trace, grid_acc, grid_sort;
 };
 
@@ -1252,7 +1252,8 @@ void with_lights(int lights, F f) {
 
 // Grid sizes for the stage kernels: persistent grids of resident blocks.
 // block_size (0 = defaults: 256 for raygen and accumulate, shade_threads for
-// the forward shade, 128 for the traces) sets them all, capped at those.
+// the forward shade) sets those, capped at the defaults. The traces always take
+// PYRE_TRACE_THREADS: their shared memory is sized for that many.
 template <bool BATCH>
 Launch make_launch(pyre_ctx* ctx, const DevScene& S, uint32_t block_size, int width) {
     Launch L;
@@ -1262,17 +1263,16 @@ Launch make_launch(pyre_ctx* ctx, const DevScene& S, uint32_t block_size, int wi
         const int b = (int)std::max(32u, std::min(256u, block_size / 32 * 32));
         L.block_stage = b;
         L.block_shade = std::min(b, L.block_shade);
-        L.block_trace = std::min(b, 128);
     }
     L.grid_raygen = grid_for(ctx, k_raygen<BATCH>, L.block_stage);
     with_lights<BATCH>(L.lights, [&](auto l) { L.grid_shade = grid_for(ctx, k_shade<BATCH, false, l()>, L.block_shade); });
-    L.grid_extend = width == 8 ? grid_for(ctx, k_extend<BATCH, 8>, L.block_trace)
-                    : width == 4 ? grid_for(ctx, k_extend<BATCH, 4>, L.block_trace)
-                                 : grid_for(ctx, k_extend<BATCH, 2>, L.block_trace);
-    L.grid_shadow = width == 8 ? grid_for(ctx, k_shadow<BATCH, 8>, L.block_trace)
-                    : width == 4 ? grid_for(ctx, k_shadow<BATCH, 4>, L.block_trace)
-                                 : grid_for(ctx, k_shadow<BATCH, 2>, L.block_trace);
-    L.grid_trace = grid_for(ctx, k_trace<BATCH>, L.block_trace);
+    L.grid_extend = width == 8 ? grid_for(ctx, k_extend<BATCH, 8>, PYRE_TRACE_THREADS)
+                    : width == 4 ? grid_for(ctx, k_extend<BATCH, 4>, PYRE_TRACE_THREADS)
+                                 : grid_for(ctx, k_extend<BATCH, 2>, PYRE_TRACE_THREADS);
+    L.grid_shadow = width == 8 ? grid_for(ctx, k_shadow<BATCH, 8>, PYRE_TRACE_THREADS)
+                    : width == 4 ? grid_for(ctx, k_shadow<BATCH, 4>, PYRE_TRACE_THREADS)
+                                 : grid_for(ctx, k_shadow<BATCH, 2>, PYRE_TRACE_THREADS);
+    L.grid_trace = grid_for(ctx, k_trace<BATCH>, PYRE_TRACE_THREADS);
     if (!BATCH && !block_size && width == 2)
         with_lights<false>(L.lights, [&](auto l) { L.blocks_small = grid_for(ctx, k_wave_small<l()>, 128); });
     L.grid_acc = BATCH ? grid_for(ctx, k_accumulate_batch, L.block_stage) : grid_for(ctx, k_accumulate, L.block_stage);
@@ -1300,16 +1300,16 @@ enum { STAGE_EXTEND = 0, STAGE_SHADE = 1, STAGE_SHADOW = 2, STAGE_OTHER = 3, STA
 template <bool BATCH>
 void launch_extend(cudaStream_t st, const Launch& Lc, const DevScene& S, const PathSoA& P, const WaveParams& W,
                    uint32_t d) {
-    if (W.bvh_width == 8) k_extend<BATCH, 8><<<Lc.grid_extend, Lc.block_trace, 0, st>>>(S, P, W, d);
-    else if (W.bvh_width == 4) k_extend<BATCH, 4><<<Lc.grid_extend, Lc.block_trace, 0, st>>>(S, P, W, d);
-    else k_extend<BATCH, 2><<<Lc.grid_extend, Lc.block_trace, 0, st>>>(S, P, W, d);
+    if (W.bvh_width == 8) k_extend<BATCH, 8><<<Lc.grid_extend, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
+    else if (W.bvh_width == 4) k_extend<BATCH, 4><<<Lc.grid_extend, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
+    else k_extend<BATCH, 2><<<Lc.grid_extend, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
 }
 template <bool BATCH>
 void launch_shadow(cudaStream_t st, const Launch& Lc, const DevScene& S, const PathSoA& P, const WaveParams& W,
                    uint32_t d) {
-    if (W.bvh_width == 8) k_shadow<BATCH, 8><<<Lc.grid_shadow, Lc.block_trace, 0, st>>>(S, P, W, d);
-    else if (W.bvh_width == 4) k_shadow<BATCH, 4><<<Lc.grid_shadow, Lc.block_trace, 0, st>>>(S, P, W, d);
-    else k_shadow<BATCH, 2><<<Lc.grid_shadow, Lc.block_trace, 0, st>>>(S, P, W, d);
+    if (W.bvh_width == 8) k_shadow<BATCH, 8><<<Lc.grid_shadow, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
+    else if (W.bvh_width == 4) k_shadow<BATCH, 4><<<Lc.grid_shadow, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
+    else k_shadow<BATCH, 2><<<Lc.grid_shadow, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
 }
 
 // Traces the shadow rays of depth d and, unless it is the last, the extend rays
@@ -1322,7 +1322,7 @@ void launch_traces(pyre_ctx* ctx, const Launch& Lc, const DevScene& S, const Pat
     cudaStream_t st = ctx->stream;
     const bool next = d + 1 < W.max_depth;
     if (next && one_trace_launch(ctx, W)) {
-        k_trace<BATCH><<<Lc.grid_trace, Lc.block_trace, 0, st>>>(S, P, W, d);
+        k_trace<BATCH><<<Lc.grid_trace, PYRE_TRACE_THREADS, 0, st>>>(S, P, W, d);
         return;
     }
     if (W.ns > 0) {
