@@ -265,7 +265,9 @@ typedef struct pyre_render_params {
     uint32_t crop[4];                /* x0, y0, x1, y1; all zero = whole image */
     uint32_t env_sampling;           /* PYRE_ENV_ALIAS or PYRE_ENV_CDF */
     uint32_t wave_paths;             /* paths in flight per wave; 0 = automatic (what a quarter
-                                        of the free device memory holds, 8 Mi to 128 Mi) */
+                                        of the free device memory holds, 8 Mi to 128 Mi; in a
+                                        batch of several jobs with host films at most an
+                                        eighth of its samples or 32 Mi) */
     uint32_t block_size;             /* threads per block of the stage kernels (at most 256;
                                         192 for the forward shade of a scene with an
                                         environment), 0 = those. The traversals always

@@ -1670,6 +1670,7 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
     std::vector<DevJob> dj(n_jobs);
     uint64_t total_pix = 0, total_samples = 0, max_npix = 0;
     uint32_t max_depth = 0;
+    bool host_films = false;
     for (uint32_t j = 0; j < n_jobs; ++j) {
         const pyre_batch_job& jb = jobs[j];
         const std::string tag = "batch job " + std::to_string(j) + ": ";
@@ -1694,6 +1695,7 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
         d.light_count = scene->part_light[2 * jb.part + 1];
         d.acc_base = (uint32_t)total_pix;
         d.inv_spp = 1.0f / (float)(jb.spp_end - jb.spp_begin);
+        host_films = host_films || jb.film.mem == PYRE_MEM_HOST;
         total_pix += d.npix;
         total_samples += (uint64_t)d.npix * (jb.spp_end - jb.spp_begin);
         max_npix = std::max<uint64_t>(max_npix, d.npix);
@@ -1702,16 +1704,20 @@ extern "C" int pyre_render_batch(pyre_ctx* ctx, const pyre_scene* scene, const p
     if (total_pix > 0x7fffffffull) return set_error(ctx, PYRE_ERR_INVALID, "pyre_render_batch: too many pixels");
 
     // ---- wave plan: jobs packed in order, each job's samples in order
-    // Automatic capacity: an eighth of the batch, from 32 Mi paths up to what the
-    // memory gives. A job's film is copied to the caller while later waves
-    // render, and nothing hides the copies of the last wave. On 40 views (318 M
-    // samples, 830 MB of host films) waves of 128 / 64 / 32 / 16 Mi paths took 213.6 /
-    // 211.9 / 214.8 / 220.5 ms on the device; the call took 217 ms with 128 Mi
-    // where the films' pages take the copies at 170 GB/s and 270 to 340 where
-    // they are fragmented and take them at a tenth of that.
+    // Automatic capacity: what the memory gives, and an eighth of the batch (from 32
+    // Mi paths up) where several jobs have host films. A job's film is copied to the
+    // caller while later waves render, and nothing hides the copies of the last
+    // wave. On 40 views (318 M samples, 830 MB of host films) waves of 128 / 64 / 32 /
+    // 16 Mi paths took 213.6 / 211.9 / 214.8 / 220.5 ms on the device; the call took
+    // 217 ms with 128 Mi where the films' pages take the copies at 170 GB/s and 270
+    // to 340 where they are fragmented and take them at a tenth of that. With device
+    // films, or one job, smaller waves only cost: 1920x1080 at 64 spp 50.4 ms in one
+    // wave, 52.2 in four; 8 views of 512x512 at 64 spp 74.6 and 75.9.
     uint64_t cap = wave_paths;
-    if (!cap) cap = std::min(default_wave_paths(ctx, scene->part_light_max, true, false, total_samples),
-                             std::max<uint64_t>((uint64_t)32 << 20, total_samples / 8));
+    if (!cap) {
+        cap = default_wave_paths(ctx, scene->part_light_max, true, false, total_samples);
+        if (n_jobs > 1 && host_films) cap = std::min(cap, std::max<uint64_t>((uint64_t)32 << 20, total_samples / 8));
+    }
     cap = std::min<uint64_t>(std::max<uint64_t>(cap, max_npix), (uint64_t)1 << 31);
     std::vector<DevSeg> segs;
     std::vector<DevWave> waves;
