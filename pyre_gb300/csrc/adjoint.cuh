@@ -321,10 +321,11 @@ struct GradTerms {
 };
 
 // Adds every lane's terms. With all 32 lanes converged, the lanes holding the
-// same material (or the same footprint) are summed with full-warp butterflies
-// (FP64 for materials), for up to PYRE_FLUSH_ROUNDS keys per kind that more
-// than one lane holds, and one lane adds each sum; every other lane adds its
-// own terms. A warp that is not converged adds lane by lane.
+// same material (or the same footprint) are summed over the warp, for up to
+// PYRE_FLUSH_ROUNDS keys per kind that more than one lane holds: a material's
+// six parameters with warp_sum6, whose sums six lanes add side by side, a
+// footprint with FP32 butterflies, whose sums one lane adds. Every other lane
+// adds its own terms. A warp that is not converged adds lane by lane.
 __device__ __forceinline__ void warp_flush(const DevScene& S, float* env_grad, double* mat_grad, const GradSmem& G,
                                            const GradTerms& t) {
     const unsigned FULL = 0xffffffffu;

@@ -263,8 +263,10 @@ __global__ void k_slot_normals(float4* __restrict__ tris, const uint32_t* __rest
 // device_scene.cuh, "binary traversal"). Nodes below top_base belong to
 // instance BVHs, the others to the top level. The last triangle of each leaf
 // gets its mark. An empty child (the second of a one-leaf BVH) becomes a LEAVE
-// entry, which does nothing there, behind a box that no ray meets unless its
-// direction is exactly along (1, 2, 4).
+// entry behind a box far out along (1, 2, 4). Few rays meet that box (those
+// heading exactly there, or with directions so short that every slab overflows),
+// and for those LEAVE is harmless: it is popped after the node's leaf, when the
+// lane has nothing left to do in the instance.
 __global__ void k_pack_nodes(GpuNode* __restrict__ nodes, uint32_t n_nodes, uint32_t top_base,
                              const DevInstance* __restrict__ inst, float4* __restrict__ tris) {
     enum { INTERIOR, LEAF, ENTRY, EMPTY };

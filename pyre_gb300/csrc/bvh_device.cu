@@ -32,7 +32,7 @@
 // The host launches several levels before it asks how many nodes are open, and
 // all arrays share one allocation (BuildWorkspace). Bound by launches: a
 // level is 8 kernels of 3 to 20 us. From and to host arrays, 300,007 triangles
-// take 1.80 ms and 1.3 M 5.3 ms; 13 kernels and a synchronisation per level down
+// take 1.82 ms and 1.3 M 5.2 ms; 13 kernels and a synchronisation per level down
 // to single primitives, with some 35 allocations per build, took 7.6 and 17.4.
 #include <cuda_runtime.h>
 

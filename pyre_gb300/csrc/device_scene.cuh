@@ -77,7 +77,7 @@ struct DevEnv {
 };
 
 struct DevScene {
-    const float4* nodes;   // GpuNode as 4 float4
+    const float4* nodes;   // trace nodes, 4 float4 each; for the wide traversals the top level's GpuNodes
     const float4* tris;
     const DevInstance* inst;
     uint32_t n_inst;

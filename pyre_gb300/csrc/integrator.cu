@@ -1,7 +1,7 @@
 // integrator.cu — wavefront path tracer and ray-query kernels for sm_103a.
 //
 // One render = waves of paths. A wave holds K samples of every pixel of the
-// crop, tile by tile (path_sample), and the film sums each pixel's samples in
+// crop, tile by tile (tile_pixel), and the film sums each pixel's samples in
 // sample order like the CLI loop (crates/pyre-cli/src/main.rs:260-285). Each
 // wave runs
 //   raygen -> [extend -> shade -> shadow] x max_depth -> accumulate
@@ -261,8 +261,8 @@ __global__ void k_wave_end(WaveCtl* ctl, uint32_t max_depth, const int* error_fl
 // 64 spp, against samples outermost (each sample sweeping the whole image):
 // 152.7 against 162.0 ms (extend 81.0 against 87.9, shadow 30.8 against 32.9,
 // shade 38.1 against 38.9); the reference's Cornell preset at 800x600, 16 spp
-// 8.59 against 8.77 ms. Both sides' traversals are bound by instruction issue
-// and load latency; this shortens the loads.
+// 8.59 against 8.77 ms (with scalar slab tests, bound by instruction issue and
+// load latency). Nearby rays shorten the loads.
 #define PYRE_TILE_W 8u
 #define PYRE_TILE_H 4u
 struct TilePixel {
